@@ -278,11 +278,53 @@ int fill_halo(sp_handle* H, int which, int inst, int f) {
                      : fill_halo_t<double>(H, which, inst, f);
 }
 
+// some side holds a constant, which the step kernels never write
+bool has_walls(const sp_handle* H) {
+  for (int s = 0; s < 2 * H->dim; ++s)
+    if (H->d.boundary[s] != SP_PERIODIC) return true;
+  return false;
+}
+
 // after new interior values: the halo of the current buffer, and the constant
-// (Dirichlet) halo of the other buffer, which the step kernels never write
+// (Dirichlet) halo of the other buffer; where every side is periodic a step
+// writes the whole halo of its output
 int refresh_halos(sp_handle* H, int inst, int f) {
-  if (int rc = fill_halo(H, H->cur ^ 1, inst, f)) return rc;
+  if (has_walls(H))
+    if (int rc = fill_halo(H, H->cur ^ 1, inst, f)) return rc;
   return fill_halo(H, H->cur, inst, f);
+}
+
+// interiors of `count` instances from instance `inst` on (equal extents, one
+// after another) to or from a dense device array, in stream order
+template <class T, bool TO_FIELD>
+int copy_dense_t(sp_handle* H, int inst, int count, int field, void* dense) {
+  const InstGeo& g = H->geo[inst];
+  sp::CopyGeo p{(long long)H->nf * (long long)g.felems, g.pitch, g.plane, g.n[0], g.n[1], g.n[2],
+                H->h[0], H->h[1], H->h[2], 0, 1};
+  // 16-byte accesses: a field's rows start on 16 bytes (its x halo and pitch
+  // are whole 16-byte units), so the dense rows and the extent decide
+  const bool wide = g.n[0] * sizeof(T) % 16 == 0 && reinterpret_cast<uintptr_t>(dense) % 16 == 0;
+  const int nv = wide ? int(g.n[0] * sizeof(T) / 16) : g.n[0];
+  const int bx = nv <= 8 ? 8 : nv <= 16 ? 16 : 32;
+  // four rows per thread where that still gives every SM several CTAs
+  const long long all = (long long)g.n[1] * g.n[2] * count * bx / sp::COPY_NT;
+  p.rows = all >= 32LL * H->sms ? 4 : 1;
+  const int rows = sp::COPY_NT / bx * p.rows;
+  p.groups = (g.n[1] + rows - 1) / rows;
+  const long long blocks = (long long)p.groups * g.n[2] * count;
+  auto kern = wide ? sp::k_batch_copy<T, 16, TO_FIELD> : sp::k_batch_copy<T, sizeof(T), TO_FIELD>;
+  SP_CUDA(H, sp::launch_pdl(kern, dim3(unsigned(blocks)), sp::COPY_NT, 0, H->stream,
+                            reinterpret_cast<T*>(field_base(H, H->cur, inst, field)),
+                            static_cast<T*>(dense), p, bx));
+  return SP_OK;
+}
+
+int copy_dense(sp_handle* H, int inst, int count, int field, void* dense, bool to_field) {
+  if (H->esz == 4)
+    return to_field ? copy_dense_t<float, true>(H, inst, count, field, dense)
+                    : copy_dense_t<float, false>(H, inst, count, field, dense);
+  return to_field ? copy_dense_t<double, true>(H, inst, count, field, dense)
+                  : copy_dense_t<double, false>(H, inst, count, field, dense);
 }
 
 int validate(const sp_desc* d, std::string& why) {
@@ -682,8 +724,29 @@ cudaMemcpy3DParms interior_copy(sp_handle* H, int which, int inst, int field, vo
   return p;
 }
 
+// whether a kernel on this handle's device may read and write `p` as values:
+// plain device memory of the current device, aligned to the values (a copy
+// engine also takes what this refuses)
+bool kernel_copyable(const sp_handle* H, const void* p) {
+  cudaPointerAttributes at{};
+  int dev = -1;
+  if (reinterpret_cast<uintptr_t>(p) % H->esz != 0) return false;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == dev;
+}
+
+// One instance's interior to or from device memory takes the copy kernel: an
+// ensemble reads its members out one call at a time, and a strided
+// device-to-device cudaMemcpy3DAsync costs about 6 us each back to back.
 int upload(sp_handle* H, int inst, int field, const void* src, size_t bytes, cudaMemcpyKind k) {
   if (int rc = check_field(H, inst, field, bytes)) return rc;
+  if (k == cudaMemcpyDeviceToDevice && kernel_copyable(H, src)) {
+    if (int rc = copy_dense(H, inst, 1, field, const_cast<void*>(src), true)) return rc;
+    return refresh_halos(H, inst, field);
+  }
   cudaMemcpy3DParms p = interior_copy(H, H->cur, inst, field, const_cast<void*>(src), true, k);
   SP_CUDA(H, cudaMemcpy3DAsync(&p, H->stream));
   return refresh_halos(H, inst, field);
@@ -692,6 +755,8 @@ int upload(sp_handle* H, int inst, int field, const void* src, size_t bytes, cud
 int download(sp_handle* H, int which, int inst, int field, void* dst, size_t bytes,
              cudaMemcpyKind k, bool wait) {
   if (int rc = check_field(H, inst, field, bytes)) return rc;
+  if (k == cudaMemcpyDeviceToDevice && which == H->cur && kernel_copyable(H, dst))
+    return copy_dense(H, inst, 1, field, dst, false);
   cudaMemcpy3DParms p = interior_copy(H, which, inst, field, dst, false, k);
   SP_CUDA(H, cudaMemcpy3DAsync(&p, H->stream));
   if (wait) return check_err_flag(H);
@@ -866,15 +931,11 @@ int batch_copy_t(sp_handle* H, int field, void* dense, size_t bytes, bool to_fie
   const long long total = (long long)H->batch * g.sites();
   if (bytes != size_t(total) * sizeof(T))
     return fail(H, SP_EINVAL, "byte count does not match batch x interior size");
-  const int blocks = int(std::min<long long>(H->sms * 8LL, (total + 255) / 256));
-  sp::k_batch_copy<T><<<blocks, 256, 0, H->stream>>>(
-      reinterpret_cast<T*>(field_base(H, H->cur, 0, field)), (long long)H->nf * g.felems,
-      g.pitch, g.plane, g.n[0], g.n[1], g.n[2], H->h[0], H->h[1], H->h[2],
-      static_cast<T*>(dense), total, to_field ? 1 : 0);
-  SP_CUDA(H, cudaGetLastError());
+  if (int rc = copy_dense(H, 0, H->batch, field, dense, to_field)) return rc;
   if (!to_field) return SP_OK;
   // as refresh_halos, for every instance at once
-  if (int rc = fill_halo_batch_t<T>(H, H->cur ^ 1, field)) return rc;
+  if (has_walls(H))
+    if (int rc = fill_halo_batch_t<T>(H, H->cur ^ 1, field)) return rc;
   return fill_halo_batch_t<T>(H, H->cur, field);
 }
 }  // namespace

@@ -3,8 +3,6 @@
  */
 #pragma once
 
-#include <utility>
-
 #include "sp_ch.cuh"
 #include "sp_chrow.cuh"
 #include "sp_row.cuh"
@@ -14,25 +12,6 @@
 #include "sp_registry.h"
 
 namespace sp {
-
-// Launches a step kernel with programmatic stream serialization: its grid may
-// start while the previous kernel in the stream drains.  Every step kernel
-// calls pdl_enter() before its first global access.
-template <class... KArgs, class... Args>
-cudaError_t launch_step_kernel(void (*kern)(KArgs...), dim3 grid, int nt, size_t smem,
-                               cudaStream_t s, Args&&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
 
 template <class MF>
 using model_of = decltype(MF{}());
@@ -47,7 +26,7 @@ struct Entry3 {
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(K::SMEM));
     if (attr != cudaSuccess) return attr;
     const M m = MF{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const StepParams<T>*>(prm), m);
   }
   static int occupancy() {
@@ -75,7 +54,7 @@ struct EntryCh3 {
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(K::SMEM));
     if (attr != cudaSuccess) return attr;
     const M m = MF{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const StepParams<T>*>(prm), m);
   }
   static int occupancy() {
@@ -110,7 +89,7 @@ struct EntryChRow {
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(K::SMEM));
     if (attr != cudaSuccess) return attr;
     const M m = MF{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const StepParams<float>*>(prm), m);
   }
   static int occupancy() {
@@ -148,7 +127,7 @@ struct EntryRow {
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(K::SMEM));
     if (attr != cudaSuccess) return attr;
     const M m = MF{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const StepParams<float>*>(prm), m);
   }
   static int occupancy() {
@@ -180,7 +159,7 @@ struct Entry2 {
     if (attr != cudaSuccess) return attr;
     const M0 m0 = MF0{}();
     const M1 m1 = MF1{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const Step2Params<T>*>(prm), m0, m1);
   }
   static int occupancy() {
@@ -210,7 +189,7 @@ struct Entry2T {
     if (attr != cudaSuccess) return attr;
     const M0 m0 = MF0{}();
     const M1 m1 = MF1{}();
-    return launch_step_kernel(kern, grid, K::NT, K::SMEM, s,
+    return launch_pdl(kern, grid, K::NT, K::SMEM, s,
                               *static_cast<const Step2Params<T>*>(prm), m0, m1);
   }
   static int occupancy() {
