@@ -1112,7 +1112,31 @@ int launch_strip(StripParams p, int* err, cudaStream_t s, int smax) {
 }  // namespace conv
 }  // namespace sp
 
+#include "sp_flow.cuh"
+
 namespace {
+// the persistent kernel (sp_flow.cuh) where it can run: input channels in
+// whole stages, and shared memory for the weights and two strips; SP_EINVAL
+// otherwise
+int flow_fwd(const sp::conv::FlowParams& p, int* err, cudaStream_t s) {
+  using namespace sp::conv;
+  if (p.cin % FL_CB != 0) return SP_EINVAL;
+  int P;
+  auto fits = [&](int MT, int BN) { return flow_stages(MT * 128, BN, p.cin, p.wid, &P) >= 2; };
+  // the largest tile that leaves room for two strips: a strip's reach beyond
+  // its tile (two rows) is gathered again by the next tile
+  if (p.cout == 32) {
+    if (fits(8, 32)) return launch_flow<32, 8>(p, err, s);
+    if (fits(4, 32)) return launch_flow<32, 4>(p, err, s);
+  } else if (p.cout == 64) {
+    if (fits(4, 64)) return launch_flow<64, 4>(p, err, s);
+    if (fits(2, 64)) return launch_flow<64, 2>(p, err, s);
+  } else if (p.cout % 128 == 0) {
+    if (fits(2, 128)) return launch_flow<128, 2>(p, err, s);
+  }
+  return SP_EINVAL;
+}
+
 int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const void* res, void* z,
               void* a, int n, int h, int w_, int cin, int cout, void* stream, int up) {
   using namespace sp::conv;
@@ -1129,6 +1153,16 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
   if ((long long)n * (h + 2) * (w_ + 2) + 4LL * (w_ + 3) + 4096 >= (1LL << 31)) return SP_EINVAL;
   int* err = tc_error_flag();
   if (!err) return SP_ENOMEM;
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!getenv("SP_STRIP_SHAPE")) {
+    const auto al = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 32 == 0; };
+    FlowParams f{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), bias,
+                 static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(z),
+                 static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout, 0, 0, 0, up,
+                 al(res) && al(z) && al(a)};
+    const int rc = flow_fwd(f, err, s);
+    if (rc != SP_EINVAL) return rc;
+  }
   const int bn = cout == 32 ? 32 : cout == 64 ? 64 : 128;
   // CTA shape by layer class, from timing every shape on the jump network's
   // layers (256 samples, 256^2 .. 32^2): narrow outputs gain from more,
@@ -1158,7 +1192,6 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
       smax = c;
     }
   }
-  const cudaStream_t s = static_cast<cudaStream_t>(stream);
   k_tile_weights<<<256, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(w),
                                       static_cast<__nv_bfloat16*>(wt), cin, cout, bn, cb);
   if (cudaGetLastError() != cudaSuccess) return SP_ECUDA;

@@ -1,0 +1,426 @@
+/*
+ * sp_flow.cuh -- the 3x3 circular convolution (forward and data gradient) as a
+ * persistent tcgen05 kernel with the weights resident in shared memory.  No
+ * counterpart in SymPhas.
+ *
+ * Same operand layout as k_conv3x3_strip (sp_conv.cu): the input is staged as
+ * a strip of circularly padded positions, chunk-major (one 16-byte row per
+ * position and 8-channel chunk), so the nine taps are nine start addresses of
+ * one staged strip.  What differs:
+ *
+ *   - one CTA per SM walks over the tiles (MT x 128 positions each); the
+ *     weights of its BN output channels are gathered once per CTA, straight
+ *     from [cout][3][3][cin] (no re-tiling launch);
+ *   - gather, MMAs and epilogue of different tiles overlap: eight producer
+ *     warps fill a ring of strips (32 input channels each), one thread issues
+ *     the MMAs into one of two tensor-memory accumulators, sixteen warps empty
+ *     the other;
+ *   - a warp gathers 8 positions x 4 chunks per copy: whole 64-byte segments
+ *     of global memory, 128-byte runs of shared memory (16-byte pieces of
+ *     different sectors, two lanes a position, read every sector twice); the
+ *     epilogue's arithmetic is packed FP32x2 and its stores are 32 bytes a lane.
+ */
+#pragma once
+
+namespace sp {
+namespace conv {
+
+constexpr int FL_PROD = 256, FL_EPI = 512;       // producer and epilogue threads
+constexpr int FL_NT = FL_PROD + 32 + FL_EPI;     // and the MMA warp
+constexpr int FL_CB = 32, FL_CH = FL_CB / 8;     // input channels per stage
+constexpr int FL_SMEM = 227 * 1024 - 1024;       // for weights and strips
+constexpr int FL_SMAX = 4;                       // stages of the ring
+
+struct FlowParams {
+  const __nv_bfloat16* x;    // [N][H][W][Cin]
+  const __nv_bfloat16* w;    // [Cout][3][3][Cin]
+  const float* bias;         // [Cout] or null
+  const __nv_bfloat16* res;  // [N][H][W][Cout] or null
+  __nv_bfloat16* z;          // pre-activation out, or null
+  __nv_bfloat16* a;          // gelu(z) out, or null
+  int n, h, wid, cin, cout;
+  int P, S;                  // positions of a strip; stages
+  int tiles;
+  int up;                    // 1: x is [N][H/2][W/2][Cin], read nearest-up-sampled
+  int wide;                  // outputs and residual allow 32-byte accesses
+};
+
+// a shared-memory descriptor as base (layout) plus start address: the start is
+// the low 14 bits in 16-byte units, so an offset is one 32-bit addition
+__device__ __forceinline__ uint64_t desc_at(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma_go(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                        uint32_t idesc) {
+  if constexpr (ACCUMULATE)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc));
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc));
+}
+
+// one arrival for a warp (an arrival per thread serialises in shared memory:
+// 512 of them a tile cost more than the tile's MMAs)
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0)
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+struct U8 {
+  uint32_t v[8];
+};
+__device__ __forceinline__ void st_32b(void* p, const U8& d, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(d.v[0]),
+                 "r"(d.v[1]), "r"(d.v[2]), "r"(d.v[3]), "r"(d.v[4]), "r"(d.v[5]), "r"(d.v[6]),
+                 "r"(d.v[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(d.v[0], d.v[1], d.v[2], d.v[3]);
+    reinterpret_cast<uint4*>(p)[1] = make_uint4(d.v[4], d.v[5], d.v[6], d.v[7]);
+  }
+}
+__device__ __forceinline__ U8 ld_32b(const void* p, bool wide) {
+  U8 d;
+  if (wide) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(d.v[0]), "=r"(d.v[1]), "=r"(d.v[2]), "=r"(d.v[3]), "=r"(d.v[4]),
+                   "=r"(d.v[5]), "=r"(d.v[6]), "=r"(d.v[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+    d = U8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+  }
+  return d;
+}
+__device__ __forceinline__ uint32_t bf2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float2 f2bf(uint32_t u) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+}
+// gelu() of two values (the same function, packed)
+__device__ __forceinline__ float2 gelu2(float2 z) {
+  const float2 q = __fmul2_rn(z, z);
+  const float2 c = __ffma2_rn(q, make_float2(0.7978845608028654f * 0.044715f,
+                                             0.7978845608028654f * 0.044715f),
+                              make_float2(0.7978845608028654f, 0.7978845608028654f));
+  const float2 u = __fmul2_rn(z, c);
+  const float2 h = __fmul2_rn(z, make_float2(0.5f, 0.5f));
+  return __ffma2_rn(h, make_float2(tanh_fast(u.x), tanh_fast(u.y)), h);
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr));
+}
+
+// A padded position: image, row and column of the (H + 2) x (W + 2) grid,
+// advanced by a fixed number of positions without divisions.
+struct PadPos {
+  int n, y, x;
+  __device__ __forceinline__ void step(int sy, int sx, int W2, int H2) {
+    x += sx;
+    y += sy;
+    if (x >= W2) {
+      x -= W2;
+      ++y;
+    }
+    while (y >= H2) {
+      y -= H2;
+      ++n;
+    }
+  }
+};
+
+template <int BN, int MT>
+struct FlowTile {
+  static constexpr int M = MT * 128;   // positions per tile
+  static constexpr int ACC = MT * BN;  // tensor-memory columns of one accumulator
+  static_assert(2 * ACC <= 512 && (2 * ACC & (2 * ACC - 1)) == 0 && 2 * ACC >= 32, "columns");
+  static_assert(BN % 32 == 0 && BN <= 128 && MT % 2 == 0, "tile");
+};
+
+template <int BN, int MT>
+__global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, int* err) {
+  using TT = FlowTile<BN, MT>;
+  constexpr int M = TT::M, ACC = TT::ACC;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int S = p.S, P = p.P, STAGE = FL_CH * P * 16;
+  const int kch = p.cin / 8;  // 8-channel chunks of the input
+  const int nkb = p.cin / FL_CB;
+  unsigned char* const wsm = smem;  // [9 * kch chunks][BN rows][16 B]
+  unsigned char* const ring = smem + 9 * kch * BN * 16;
+  float* const bsm = reinterpret_cast<float*>(ring + S * STAGE);  // [BN] bias
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(bsm + BN);
+  uint64_t *const full = bars, *const empty = bars + FL_SMAX, *const tfull = bars + 2 * FL_SMAX,
+           *const tempty = tfull + 2, *const done = tempty + 2;
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int W2 = p.wid + 2, H2 = p.h + 2;
+  const uint32_t W2u = uint32_t(W2), HW2u = uint32_t(W2) * uint32_t(H2);
+  const int co0 = blockIdx.y * BN;
+  constexpr int MMA_WARP = FL_PROD / 32;
+
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(2 * ACC));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      tma::mbar_init(&full[s], FL_PROD / 32);
+      tma::mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      tma::mbar_init(&tfull[b], 1);
+      tma::mbar_init(&tempty[b], FL_EPI / 32);
+    }
+    tma::mbar_init(done, 1);
+    tma::fence_barrier_init();
+  }
+  // the weights, K-major without swizzle: [tap * kch + chunk][output channel]
+  for (int i = tid; i < 9 * kch * BN; i += FL_NT) {
+    const int co = i % BN, kc = i / BN;
+    cp_async16(wsm + i * 16, p.w + ((long long)(co0 + co) * 9 * kch + kc) * 8, true);
+  }
+  for (int i = tid; i < BN; i += FL_NT) bsm[i] = p.bias ? p.bias[co0 + i] : 0.f;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  tma::fence_proxy_async();  // generic-proxy writes, read by the tensor core
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  bool bad = false;
+
+  if (warp < MMA_WARP) {
+    // ---- producers: a warp copies 8 positions x 4 chunks at a time; lane:
+    // position lp, chunk j
+    const int j = lane >> 3, lp = warp * 8 + (lane & 7);
+    constexpr int STEP = FL_PROD / FL_CH;
+    const int sy = STEP / W2, sx = STEP - sy * W2;
+    int s = 0;
+    uint32_t ph = 1;  // a fresh barrier passes the wait for the phase before its first
+    for (int tile = blockIdx.x; tile < p.tiles && !bad; tile += gridDim.x) {
+      // strip position 0 is output position tile * M - (W2 + 1); counted from
+      // one image earlier, so that it is not negative
+      const uint32_t u = uint32_t(tile) * M + HW2u - uint32_t(W2 + 1) + uint32_t(lp);
+      const uint32_t nn = u / HW2u, r = u - nn * HW2u, yq = r / W2u;
+      const PadPos start{int(nn) - 1, int(yq), int(r - yq * W2u)};
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!tma::mbar_wait(&empty[s], ph)) {
+          bad = true;
+          break;
+        }
+        unsigned char* dst = ring + s * STAGE + (j * P + lp) * 16;
+        const __nv_bfloat16* const xc = p.x + kb * FL_CB + j * 8;
+        PadPos q = start;
+#pragma unroll 4
+        for (int pos = lp; pos < P; pos += STEP) {
+          int yy = q.y - 1, xx = q.x - 1;
+          yy += yy < 0 ? p.h : 0;
+          yy -= yy >= p.h ? p.h : 0;
+          xx += xx < 0 ? p.wid : 0;
+          xx -= xx >= p.wid ? p.wid : 0;
+          const bool ok = unsigned(q.n) < unsigned(p.n);
+          const int off = p.up ? ((q.n * (p.h >> 1) + (yy >> 1)) * (p.wid >> 1) + (xx >> 1)) * p.cin
+                               : ((q.n * p.h + yy) * p.wid + xx) * p.cin;
+          cp_async16(dst, xc + (ok ? off : 0), ok);
+          dst += STEP * 16;
+          q.step(sy, sx, W2, H2);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        tma::fence_proxy_async();
+        warp_arrive(&full[s], lane);
+        if (++s == S) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+    }
+  } else if (warp == MMA_WARP) {
+    if (lane == 0) {
+      // ---- MMA issuer: per stage, for every tap and K step of 16 channels,
+      // one MMA per 128 positions
+      constexpr uint32_t idesc = umma_idesc<BN>();
+      constexpr uint32_t HI = (128u >> 4) | (1u << 14);  // 128 B between 8-row groups, version 1
+      const uint32_t alo = uint32_t(P) << 16, blo = uint32_t(BN) << 16;  // chunk strides / 16
+      const uint32_t w0 = blo + (smem_u32(wsm) >> 4), r0 = alo + (smem_u32(ring) >> 4);
+      int s = 0, it = 0;
+      uint32_t ph = 0;
+      for (int tile = blockIdx.x; tile < p.tiles && !bad; tile += gridDim.x, ++it) {
+        const int b = it & 1;
+        if (!tma::mbar_wait(&tempty[b], uint32_t((it >> 1) & 1) ^ 1u)) {
+          bad = true;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + uint32_t(b * ACC);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!tma::mbar_wait(&full[s], ph)) {
+            bad = true;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a0 = r0 + uint32_t(s * FL_CH * P);
+          const uint32_t b0 = w0 + uint32_t(kb * FL_CH * BN);
+          auto tap = [&](int t, auto first) {
+            const uint32_t at = a0 + uint32_t((t / 3) * W2 + t % 3);  // position 0 of the tap
+            const uint32_t bt = b0 + uint32_t(t * kch * BN);
+#pragma unroll
+            for (int kk = 0; kk < FL_CB / 16; ++kk) {
+              const uint64_t bd = desc_at(bt + 2 * kk * BN, HI);
+              const uint32_t ak = at + uint32_t(2 * kk * P);
+#pragma unroll
+              for (int m = 0; m < MT; ++m) {
+                if (decltype(first)::value && kk == 0)
+                  umma_go<false>(acc + uint32_t(m * BN), desc_at(ak + m * 128, HI), bd, idesc);
+                else
+                  umma_go<true>(acc + uint32_t(m * BN), desc_at(ak + m * 128, HI), bd, idesc);
+              }
+            }
+          };
+          if (kb == 0)
+            tap(0, std::true_type{});
+          else
+            tap(0, std::false_type{});
+#pragma unroll 1
+          for (int t = 1; t < 9; ++t) tap(t, std::false_type{});
+          umma_commit(&empty[s]);
+          if (++s == S) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        umma_commit(&tfull[b]);
+      }
+      // every MMA of this CTA done (also after giving up) before it leaves
+      umma_commit(done);
+      bad |= !tma::mbar_wait(done, 0);
+    }
+  } else {
+    // ---- epilogue: a warp reads lanes 32 (warp % 4) .. + 31 of units (128
+    // positions x 32 channels) g, g + G, ...
+    constexpr int UNITS = MT * BN / 32, G = FL_EPI / 128;
+    static_assert(UNITS % G == 0, "units per warp");
+    const int lq = 32 * (warp & 3), g = (warp - MMA_WARP - 1) >> 2;
+    const bool wide = p.wide != 0;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
+      const int b = it & 1;
+      bool ok = tma::mbar_wait(&tfull[b], uint32_t((it >> 1) & 1));
+      ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is warp-collective
+      if (!ok) {
+        bad = true;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int k = 0; k < UNITS / G; ++k) {
+        const int unit = g + k * G, m = unit / (BN / 32), c = unit % (BN / 32);
+        const uint32_t q = uint32_t(tile) * M + m * 128 + lq + lane;
+        const uint32_t nn = q / HW2u, r = q - nn * HW2u, yq = r / W2u;
+        const int yp = int(yq), xp = int(r - yq * W2u);
+        const bool store =
+            int(nn) < p.n && yp >= 1 && yp <= p.h && xp >= 1 && xp <= p.wid;
+        const long long o =
+            (((long long)nn * p.h + (yp - 1)) * p.wid + (xp - 1)) * p.cout + co0 + c * 32;
+        U8 rr[2];
+        if (p.res && store) {
+          rr[0] = ld_32b(p.res + o, wide);
+          rr[1] = ld_32b(p.res + o + 16, wide);
+        }
+        uint32_t v[32];
+        __syncwarp();
+        tmem_ld32(tmem + (uint32_t(lq) << 16) + uint32_t(b * ACC + m * BN + c * 32), v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (k == UNITS / G - 1) {
+          // the accumulator is in registers: it may be overwritten
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          warp_arrive(&tempty[b], lane);
+        }
+        if (store) {
+          const float4* const bias = reinterpret_cast<const float4*>(bsm + c * 32);
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            U8 zz, aa;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float4 bb = bias[hf * 4 + e];
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                float2 f = make_float2(__uint_as_float(v[hf * 16 + 4 * e + 2 * i]),
+                                       __uint_as_float(v[hf * 16 + 4 * e + 2 * i + 1]));
+                f = __fadd2_rn(f, i ? make_float2(bb.z, bb.w) : make_float2(bb.x, bb.y));
+                if (p.res) f = __fadd2_rn(f, f2bf(rr[hf].v[2 * e + i]));
+                if (p.z) zz.v[2 * e + i] = bf2(f.x, f.y);
+                if (p.a) {
+                  const float2 ge = gelu2(f);
+                  aa.v[2 * e + i] = bf2(ge.x, ge.y);
+                }
+              }
+            }
+            if (p.z) st_32b(p.z + o + hf * 16, zz, wide);
+            if (p.a) st_32b(p.a + o + hf * 16, aa, wide);
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == MMA_WARP)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(2 * ACC));
+  if (bad) atomicExch(err, 1);
+}
+
+// Shared memory of a launch with tiles of M positions and BN output channels,
+// and the stages it leaves room for (0: it does not fit).
+inline int flow_stages(int M, int BN, int cin, int wid, int* P) {
+  const int q = (M + 2 * (wid + 3) + 7) / 8 * 8;  // M positions and the taps' reach
+  *P = q;
+  const int weights = 9 * cin * BN * 2, stage = FL_CH * q * 16;
+  const int s = (FL_SMEM - weights) / stage;
+  return weights >= FL_SMEM ? 0 : s > FL_SMAX ? FL_SMAX : s;
+}
+
+template <int BN, int MT>
+int launch_flow(FlowParams p, int* err, cudaStream_t s) {
+  using TT = FlowTile<BN, MT>;
+  p.S = flow_stages(TT::M, BN, p.cin, p.wid, &p.P);
+  if (p.S < 2) return SP_EINVAL;
+  const int smem = 9 * p.cin * BN * 2 + p.S * FL_CH * p.P * 16 + 1024;
+  const cudaError_t attr =
+      cudaFuncSetAttribute(k_conv3x3_flow<BN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           227 * 1024);
+  if (attr != cudaSuccess) return SP_ECUDA;
+  const long long QN = (long long)(p.h + 2) * (p.wid + 2) * p.n;
+  p.tiles = int((QN + TT::M - 1) / TT::M);
+  const int ny = p.cout / BN, gx = sms() / ny > 0 ? sms() / ny : 1;
+  k_conv3x3_flow<BN, MT><<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)), FL_NT, smem,
+                           s>>>(p, err);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
+}
+
+}  // namespace conv
+}  // namespace sp
