@@ -453,27 +453,6 @@ int sp_conv3x3_fwd(const void* x, const void* w, const float* bias, const void* 
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 
-int sp_conv3x3_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w_, int cin,
-                     int cout, void* stream) {
-  using namespace sp::conv;
-  if (!x || !dy || !dw || n < 1 || h < 1 || w_ < 1 || cin % WM != 0 || cout % 8 != 0)
-    return SP_EINVAL;
-  const long long npix = (long long)n * h * w_;
-  if (npix >= (1LL << 31)) return SP_EINVAL;  // the kernel's pixel arithmetic is 32-bit
-  const unsigned gx = unsigned(9 * (cin / WM)), gy = unsigned((cout + WN - 1) / WN);
-  // enough pixel chunks for about four waves of CTAs
-  long long want = (long long)sms() * 8 / (gx * gy);
-  if (want < 1) want = 1;
-  long long chunk = (npix + want - 1) / want;
-  chunk = ((chunk + WK - 1) / WK) * WK;
-  if (chunk < 1024) chunk = 1024;
-  const unsigned gz = unsigned((npix + chunk - 1) / chunk);
-  WgradParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw,
-                n, h, w_, cin, cout, chunk};
-  k_conv3x3_wgrad<<<dim3(gx, gy, gz), WTH, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
-}
-
 int sp_embed_channel0_bf16(const float* psi, void* x, long long npix, int c, void* stream) {
   if (!psi || !x || npix < 1 || c < 8 || c % 8) return SP_EINVAL;
   if (reinterpret_cast<uintptr_t>(x) % 16 != 0) return SP_EINVAL;  // 16-byte stores
@@ -1224,4 +1203,34 @@ extern "C" int sp_conv3x3_fwd_strip_up2(const void* x, const void* w, void* wt, 
                                         int cin, int cout, void* stream) {
   if (h < 2 || w_ < 2 || h % 2 != 0 || w_ % 2 != 0) return SP_EINVAL;
   return strip_fwd(x, w, wt, bias, res, z, a, n, h, w_, cin, cout, stream, 1);
+}
+
+#include "sp_wgrad.cuh"
+
+extern "C" int sp_conv3x3_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w_, int cin,
+                     int cout, void* stream) {
+  using namespace sp::conv;
+  if (!x || !dy || !dw || n < 1 || h < 1 || w_ < 1 || cin % WM != 0 || cout % 8 != 0)
+    return SP_EINVAL;
+  const long long npix = (long long)n * h * w_;
+  if (npix >= (1LL << 31)) return SP_EINVAL;  // the kernel's pixel arithmetic is 32-bit
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (int* err = tc_error_flag()) {
+    WgParams t{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw,
+               n, h, w_, cin, cout, 0, 0, 0, 0, 0, reinterpret_cast<uintptr_t>(dw) % 16 == 0};
+    const int rc = wgrad_tc(t, err, s);
+    if (rc != SP_EINVAL) return rc;
+  }
+  const unsigned gx = unsigned(9 * (cin / WM)), gy = unsigned((cout + WN - 1) / WN);
+  // enough pixel chunks for about four waves of CTAs
+  long long want = (long long)sms() * 8 / (gx * gy);
+  if (want < 1) want = 1;
+  long long chunk = (npix + want - 1) / want;
+  chunk = ((chunk + WK - 1) / WK) * WK;
+  if (chunk < 1024) chunk = 1024;
+  const unsigned gz = unsigned((npix + chunk - 1) / chunk);
+  WgradParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw,
+                n, h, w_, cin, cout, chunk};
+  k_conv3x3_wgrad<<<dim3(gx, gy, gz), WTH, 0, s>>>(p);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
