@@ -299,6 +299,24 @@ int sp_embed_channel0_bf16(const float* psi, void* x, long long npix, int c, voi
  * h, w_ even, c a multiple of 8, 16-byte aligned rows): the jump network's
  * pooling at inference.  No counterpart in SymPhas. */
 int sp_avgpool2_bf16(const void* x, void* y, int n, int h, int w_, int c, void* stream);
+/* The jump network's first layer at inference: a [n][h][w_][cout] (bf16) =
+ * gelu(conv3x3 of an input whose channel 0 is the fp32 field psi [n][h][w_]
+ * rounded to bf16 and whose other channels are zero, + bias), w [cout][3][3]
+ * [cin] (only its channel 0 is read); cout a multiple of 32, a 16-byte
+ * aligned.  No counterpart in SymPhas. */
+int sp_conv3x3_in1(const float* psi, const void* w, const float* bias, void* a, int n, int h,
+                   int w_, int cin, int cout, void* stream);
+/* The network's last layer at inference: out [n][h][w_] (fp32) = channel 0 of
+ * conv3x3(x [n][h][w_][cin], w) + bias[0] (bias may be null), not rounded to
+ * bf16; cin 32 or 64, x and w 16-byte aligned.  No counterpart in SymPhas. */
+int sp_conv3x3_out1(const void* x, const void* w, const float* bias, float* out, int n, int h,
+                    int w_, int cin, void* stream);
+/* The element-wise backward of a layer: dz [npix][c] (bf16) = da * gelu'(z)
+ * (tanh form) and db [c] (fp32, or null) += the sums of dz over the pixels;
+ * with z null dz is not written and db gets the sums of da.  c a multiple of
+ * 8, at most 2048; z, da, dz 16-byte aligned.  No counterpart in SymPhas. */
+int sp_gelu_bwd_bf16(const void* z, const void* da, void* dz, float* db, long long npix, int c,
+                     void* stream);
 /* wf [cin][3][3][cout] = w [cout][3][3][cin] rotated by 180 degrees: the input
  * gradient of the convolution is sp_conv3x3_fwd(dy, wf). */
 int sp_conv3x3_flip(const void* w, void* wf, int cin, int cout, void* stream);

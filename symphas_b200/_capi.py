@@ -132,6 +132,11 @@ SIGNATURES = {
     "sp_avgpool2_bf16": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                         ctypes.c_int, _P]),
     "sp_embed_channel0_bf16": (ctypes.c_int, [_P, _P, ctypes.c_longlong, ctypes.c_int, _P]),
+    "sp_conv3x3_in1": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                      ctypes.c_int, ctypes.c_int, _P]),
+    "sp_conv3x3_out1": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                       ctypes.c_int, _P]),
+    "sp_gelu_bwd_bf16": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_longlong, ctypes.c_int, _P]),
     "sp_conv3x3_wgrad": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                         ctypes.c_int, ctypes.c_int, _P]),
     "sp_conv3x3_flip": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int, _P]),

@@ -1234,3 +1234,5 @@ extern "C" int sp_conv3x3_wgrad(const void* x, const void* dy, float* dw, int n,
   k_conv3x3_wgrad<<<dim3(gx, gy, gz), WTH, 0, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
+
+#include "sp_ends.cuh"

@@ -9,9 +9,10 @@ psi exactly as model B does.  Convolutions, their gradients and the Adam
 update run in this package's BF16 tensor-core kernels
 (sp_conv3x3_fwd_tc on tcgen05 with the accumulator in tensor memory, or
 sp_conv3x3_fwd on mma.sync; sp_conv3x3_wgrad / sp_conv3x3_flip /
-sp_adam_step; fp32 accumulation, fp32 master weights); PyTorch holds the
-tensors and does the element-wise glue (pooling, up-sampling, the loss, and
-GELU under autograd -- at inference the convolution's epilogue applies it).
+sp_adam_step; fp32 accumulation, fp32 master weights), with GELU in the
+convolutions' epilogue and its derivative in one kernel with the bias gradient;
+PyTorch holds the tensors and does the rest of the element-wise glue (the loss,
+and under autograd pooling and up-sampling).
 
 Training data are trajectories of this package's own fused FD kernel
 (model_MB_t, batch of instances in one persistent launch).  At inference each
@@ -131,16 +132,58 @@ class _Conv(torch.autograd.Function):
     def backward(ctx, dz):
         (x,) = ctx.saved_tensors
         L = ctx.layer
-        dz = dz.contiguous().bfloat16()
+        dz = _aligned(dz)
+        _ok(C.lib().sp_gelu_bwd_bf16(None, _p(dz), None, _p(L.gb), dz.numel() // L.cout, L.cout,
+                                     _s()), "sp_gelu_bwd_bf16")
+        dx = _grads(x, dz, L, ctx.needs_input_grad[0])
+        return dx, None, None, (dz if ctx.has_res else None)
+
+
+def _aligned(g):
+    """A gradient as the kernels read it: contiguous bf16 on a 16-byte boundary."""
+    g = g.contiguous().bfloat16()
+    return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
+def _grads(x, dz, L, need_dx):
+    """Accumulate the weight gradient for the pre-activation gradient dz, and
+    the data gradient (a forward convolution of the flipped weights) if needed."""
+    n, h, w, ci = x.shape
+    _ok(C.lib().sp_conv3x3_wgrad(_p(x), _p(dz), _p(L.gw), n, h, w, ci, L.cout, _s()),
+        "sp_conv3x3_wgrad")
+    if not need_dx:
+        return None
+    _ok(C.lib().sp_conv3x3_flip(_p(L.wb), _p(L.wf), ci, L.cout, _s()), "sp_conv3x3_flip")
+    dx = torch.empty_like(x)
+    _fwd(dz, L.wf, None, None, dx, None, L.cout, ci, L.wt)
+    return dx
+
+
+class _ConvGelu(torch.autograd.Function):
+    """gelu(conv3x3(x) + bias (+ res)): the convolution's epilogue writes the
+    pre-activation and the activation; backward, one kernel gives the
+    pre-activation gradient and the bias gradient."""
+
+    @staticmethod
+    def forward(ctx, x, anchor, layer, res):
         n, h, w, ci = x.shape
-        _ok(C.lib().sp_conv3x3_wgrad(_p(x), _p(dz), _p(L.gw), n, h, w, ci, L.cout, _s()),
-            "sp_conv3x3_wgrad")
-        L.gb += dz.float().sum((0, 1, 2))
-        dx = None
-        if ctx.needs_input_grad[0]:
-            _ok(C.lib().sp_conv3x3_flip(_p(L.wb), _p(L.wf), ci, L.cout, _s()), "sp_conv3x3_flip")
-            dx = torch.empty_like(x)
-            _fwd(dz, L.wf, None, None, dx, None, L.cout, ci, L.wt)
+        z = torch.empty(n, h, w, layer.cout, device="cuda", dtype=torch.bfloat16)
+        a = torch.empty_like(z)
+        _fwd(x, layer.wb, layer.b, res, z, a, ci, layer.cout, layer.wt)
+        ctx.save_for_backward(x, z)
+        ctx.layer = layer
+        ctx.has_res = res is not None
+        return a
+
+    @staticmethod
+    def backward(ctx, da):
+        x, z = ctx.saved_tensors
+        L = ctx.layer
+        da = _aligned(da)
+        dz = torch.empty_like(z)
+        _ok(C.lib().sp_gelu_bwd_bf16(_p(z), _p(da), _p(dz), _p(L.gb), z.numel() // L.cout, L.cout,
+                                     _s()), "sp_gelu_bwd_bf16")
+        dx = _grads(x, dz, L, ctx.needs_input_grad[0])
         return dx, None, None, (dz if ctx.has_res else None)
 
 
@@ -153,10 +196,10 @@ def gelu(z):
 
 
 def conv_gelu(x, layer, res=None):
-    """gelu(conv(x) + bias (+ res)); without autograd, one kernel writes the
-    activation from its epilogue."""
+    """gelu(conv(x) + bias (+ res)), the activation from the convolution's
+    epilogue; without autograd no pre-activation is kept."""
     if torch.is_grad_enabled():
-        return gelu(conv(x, layer, res))
+        return _ConvGelu.apply(x, layer.anchor, layer, res)
     n, h, w, ci = x.shape
     a = torch.empty(n, h, w, layer.cout, device="cuda", dtype=torch.bfloat16)
     _fwd(x, layer.wb, layer.b, res, None, a, ci, layer.cout, layer.wt)
@@ -224,20 +267,36 @@ class JumpNet:
     def __call__(self, psi):
         """psi [N, H, W] (fp32) -> predicted change over one jump, zero mean."""
         n, h, w = psi.shape
-        x = torch.empty(n, h, w, CIN, device="cuda", dtype=torch.bfloat16)
         src = psi.contiguous().float()
-        _ok(C.lib().sp_embed_channel0_bf16(_p(src), _p(x), n * h * w, CIN, _s()),
-            "sp_embed_channel0_bf16")
+        # at inference the first and the last layer read and write the field
+        # itself (sp_conv3x3_in1, sp_conv3x3_out1) instead of 32 channels of
+        # which one is used
+        ends = not torch.is_grad_enabled() and n * (self.ch[0] // 32) <= 65535
         skips = []
         for lvl, (a, b) in enumerate(self.enc):
-            x = conv_gelu(conv_gelu(x, a), b)
+            if lvl == 0 and ends and self.ch[0] % 32 == 0:
+                x = torch.empty(n, h, w, a.cout, device="cuda", dtype=torch.bfloat16)
+                _ok(C.lib().sp_conv3x3_in1(_p(src), _p(a.wb), _p(a.b), _p(x), n, h, w, a.cin,
+                                           a.cout, _s()), "sp_conv3x3_in1")
+            else:
+                if lvl == 0:
+                    x = torch.empty(n, h, w, CIN, device="cuda", dtype=torch.bfloat16)
+                    _ok(C.lib().sp_embed_channel0_bf16(_p(src), _p(x), n * h * w, CIN, _s()),
+                        "sp_embed_channel0_bf16")
+                x = conv_gelu(x, a)
+            x = conv_gelu(x, b)
             if lvl < len(self.enc) - 1:
                 skips.append(x)
                 x = pool2(x)
         for (a, b), s in zip(self.dec, reversed(skips)):
             x = conv_gelu_up(x, a, res=s)
             x = conv_gelu(x, b)
-        d = conv(x, self.head)[..., 0].float()
+        if ends and self.head.cin in (32, 64):
+            d = torch.empty(n, h, w, device="cuda")
+            _ok(C.lib().sp_conv3x3_out1(_p(x), _p(self.head.wb), _p(self.head.b), _p(d), n, h, w,
+                                        self.head.cin, _s()), "sp_conv3x3_out1")
+        else:
+            d = conv(x, self.head)[..., 0].float()
         d = d - d.mean((1, 2), keepdim=True)  # exact mass conservation
         return d * self.scale
 

@@ -1,0 +1,124 @@
+"""The jump network's first and last convolutions as kernels of their own, the
+element-wise backward with the bias gradient, and a layer's autograd function,
+against float64 references on the same bf16 operands: image edges (circular
+wrap, extents 1 and 2, column blocks of 64 and 62, row blocks of 32), every
+channel count of the dispatch.  Outputs stored in bf16 are within one rounding
+(2^-8 of the value) plus tanh.approx's 2^-11; fp32 sums of K bf16 products
+within K 2^-24 of the sum of magnitudes."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from symphas_b200 import _capi as C
+from symphas_b200 import surrogate as S
+
+pytestmark = pytest.mark.gpu
+
+
+def ptr(t):
+    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def conv64(x, w, b=None):
+    n, h, wd, ci = x.shape
+    out = 0
+    for t in range(9):
+        xs = torch.roll(x.double(), (1 - t // 3, 1 - t % 3), (1, 2))
+        out = out + xs.reshape(-1, ci) @ w.double()[:, t // 3, t % 3].t()
+    return (out if b is None else out + b.double()).view(n, h, wd, -1)
+
+
+SIZES = [(1, 1, 1), (2, 2, 3), (1, 33, 64), (2, 32, 65), (1, 31, 62), (1, 64, 63), (1, 5, 256)]
+
+
+@pytest.mark.parametrize("n,h,w", SIZES)
+@pytest.mark.parametrize("co", [32, 96])
+def test_first_layer(n, h, w, co):
+    torch.manual_seed(h + w)
+    psi = torch.randn(n, h, w, device="cuda")
+    wt = (torch.randn(co, 3, 3, 32, device="cuda") / 3).bfloat16()
+    b = 0.1 * torch.randn(co, device="cuda")
+    a = torch.full((n, h, w, co), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert C.lib().sp_conv3x3_in1(ptr(psi), ptr(wt), ptr(b), ptr(a), n, h, w, 32, co,
+                                  stream()) == C.SP_OK
+    want = F.gelu(conv64(psi.bfloat16()[..., None], wt[..., :1], b), approximate="tanh")
+    assert torch.allclose(a.double(), want, rtol=2.0 ** -7, atol=2e-3)
+    assert C.lib().sp_conv3x3_in1(ptr(psi), ptr(wt), ptr(b), ptr(a), n, h, w, 32, 48,
+                                  stream()) == C.SP_EINVAL
+
+
+@pytest.mark.parametrize("n,h,w", SIZES)
+@pytest.mark.parametrize("ci", [32, 64])
+def test_last_layer(n, h, w, ci):
+    torch.manual_seed(h + w)
+    x = torch.randn(n, h, w, ci, device="cuda").bfloat16()
+    wt = torch.randn(32, 3, 3, ci, device="cuda").bfloat16()
+    b = torch.randn(32, device="cuda")
+    out = torch.full((n, h, w), float("nan"), device="cuda")
+    assert C.lib().sp_conv3x3_out1(ptr(x), ptr(wt), ptr(b), ptr(out), n, h, w, ci,
+                                   stream()) == C.SP_OK
+    want = conv64(x, wt[:1], b[:1])[..., 0]
+    mag = conv64(x.abs(), wt[:1].abs())[..., 0]
+    assert ((out.double() - want).abs() <= 9 * ci * 2.0 ** -24 * (mag + 1)).all()
+    assert C.lib().sp_conv3x3_out1(ptr(x), ptr(wt), ptr(b), ptr(out), n, h, w, 16,
+                                   stream()) == C.SP_EINVAL
+
+
+@pytest.mark.parametrize("npix,c", [(1, 8), (7, 24), (1000, 32), (33, 256), (5, 2048), (70000, 64)])
+def test_gelu_backward_and_bias_gradient(npix, c):
+    torch.manual_seed(c)
+    z = (3 * torch.randn(npix, c, device="cuda")).bfloat16()
+    z[0, :4] = torch.tensor([0.0, -30.0, 30.0, 1e4])
+    da = torch.randn(npix, c, device="cuda").bfloat16()
+    dz = torch.full_like(z, float("nan"))
+    db = torch.ones(c, device="cuda")
+    assert C.lib().sp_gelu_bwd_bf16(ptr(z), ptr(da), ptr(dz), ptr(db), npix, c, stream()) == C.SP_OK
+    zr = z.double().requires_grad_()
+    F.gelu(zr, approximate="tanh").backward(da.double())
+    # the derivative in fp32 to ~2e-6 absolute, then one bf16 rounding
+    tol = 2.0 ** -8 * zr.grad.abs() + 2e-6 * da.double().abs() + 1e-30
+    assert ((dz.double() - zr.grad).abs() <= tol).all()
+    bound = npix * 2.0 ** -24 * (dz.double().abs().sum(0) + 1) + 1e-6
+    assert ((db.double() - 1 - dz.double().sum(0)).abs() <= bound).all()
+    db2 = torch.zeros(c, device="cuda")
+    assert C.lib().sp_gelu_bwd_bf16(None, ptr(da), None, ptr(db2), npix, c, stream()) == C.SP_OK
+    bound = npix * 2.0 ** -24 * (da.double().abs().sum(0) + 1) + 1e-6
+    assert ((db2.double() - da.double().sum(0)).abs() <= bound).all()
+    assert C.lib().sp_gelu_bwd_bf16(ptr(z), ptr(da), None, ptr(db), npix, c,
+                                    stream()) == C.SP_EINVAL
+
+
+@pytest.mark.parametrize("skip", [False, True])
+def test_layer_autograd(skip):
+    """conv_gelu under autograd, with an upstream gradient that does not start
+    on a 16-byte boundary."""
+    torch.manual_seed(5)
+    n, h, w, ci, co = 2, 12, 20, 32, 64
+    layer = S.ConvLayer(ci, co, torch.Generator().manual_seed(1))
+    layer.b.normal_()
+    x = torch.randn(n, h, w, ci, device="cuda").bfloat16().requires_grad_()
+    res = torch.randn(n, h, w, co, device="cuda").bfloat16().requires_grad_() if skip else None
+    buf = torch.randn(n * h * w * co + 1, device="cuda").bfloat16()
+    dy = buf[1:].view(n, h, w, co)
+    y = S.conv_gelu(x, layer, res)
+    y.backward(dy)
+    xr, wr = x.detach().double().requires_grad_(), layer.wb.double().requires_grad_()
+    br = layer.b.double().requires_grad_()
+    zr = conv64(xr, wr, br)
+    rr = res.detach().double().requires_grad_() if skip else None
+    yr = F.gelu(zr if rr is None else zr + rr, approximate="tanh")
+    yr.backward(dy.double())
+
+    def rel(a, b):
+        return float((a.double() - b).norm() / b.norm())
+
+    assert rel(y, yr) < 4e-3 and rel(x.grad, xr.grad) < 8e-3
+    assert rel(layer.gw, wr.grad) < 4e-3 and rel(layer.gb, br.grad) < 8e-3
+    if skip:
+        assert rel(res.grad, rr.grad) < 4e-3
