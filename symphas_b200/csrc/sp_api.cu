@@ -23,6 +23,7 @@
 #include "../../include/symphas_b200.h"
 #include "sp_aux.cuh"
 #include "sp_kernels.cuh"
+#include "sp_many2.cuh"
 #include "sp_registry.h"
 
 namespace sp {
@@ -46,18 +47,33 @@ const std::vector<KernelInfo>* find_kernels(const KernelKey& key) {
   auto it = table().find(tup(key));
   return it == table().end() ? nullptr : &it->second;
 }
+namespace {
+std::map<KeyT, ManyInfo>& many_table() {
+  static std::map<KeyT, ManyInfo> t;
+  return t;
+}
+}  // namespace
+void register_many(const KernelKey& key, const ManyInfo& info) { many_table()[tup(key)] = info; }
+const ManyInfo* find_many(const KernelKey& key) {
+  auto it = many_table().find(tup(key));
+  return it == many_table().end() ? nullptr : &it->second;
+}
 // the built-in kernel sets (sp_inst_exact.cu, sp_inst_fused.cu,
-// sp_inst_wide.cu); weak, so a program that compiles this runtime with only
+// sp_inst_wide.cu, sp_inst_many.cu, sp_inst_many_exact.cu); weak, so a program that compiles this runtime with only
 // its own models (the C++ front end, symphas_model.hpp) links without them
 void register_exact_kernels() __attribute__((weak));
 void register_fused_kernels() __attribute__((weak));
 void register_wide_kernels() __attribute__((weak));
+void register_many_kernels() __attribute__((weak));
+void register_many_exact_kernels() __attribute__((weak));
 void register_all_kernels() {
   static std::once_flag once;
   std::call_once(once, [] {
     if (register_exact_kernels) register_exact_kernels();
     if (register_fused_kernels) register_fused_kernels();
     if (register_wide_kernels) register_wide_kernels();
+    if (register_many_kernels) register_many_kernels();
+    if (register_many_exact_kernels) register_many_exact_kernels();
   });
 }
 
@@ -219,6 +235,50 @@ int launch_step(sp_handle* H, int rhs_only, double* partial, int steps = 1, bool
     return fail(H, SP_EINVAL, "steps per launch outside the kernel's range");
   return H->esz == 4 ? launch_step_t<float>(H, rhs_only, partial, steps, advance)
                      : launch_step_t<double>(H, rhs_only, partial, steps, advance);
+}
+
+// margin of the many-step kernel's tile along x: whole groups, and one more for
+// the sites a region is rounded out by
+int many_hx(const sp_handle* H, int steps, int R) {
+  const int w = sp::many_w(int(H->esz));
+  return (steps * R + w - 1) / w * w + w;
+}
+size_t many_smem(const sp_handle* H, int ty, int steps) {
+  return size_t(H->many->planes) * sp::MANY_PW *
+         (ty + 2 * steps * H->many->R + sp::MANY_SR - 1) * H->esz;
+}
+
+// `steps` steps in one launch of the many-step kernel
+template <class T>
+int launch_many_t(sp_handle* H, int steps) {
+  const int src = H->cur, dst = H->cur ^ 1, R = H->many->R;
+  sp::ManyParams<T> q{};
+  q.s.out = reinterpret_cast<T* const*>(H->outs_d[dst]);
+  q.s.in = reinterpret_cast<const T* const*>(H->outs_d[src]);
+  q.s.inst = static_cast<const sp::Inst2<T>*>(H->inst2_d);
+  q.s.hx = H->h[0];
+  q.s.hy = H->h[1];
+  q.s.tsteps = steps;
+  q.t.tx = H->many_tx;
+  q.t.ty = H->many_ty;
+  q.t.ntx = (H->n[0] + H->many_tx - 1) / H->many_tx;
+  q.t.hx = many_hx(H, steps, R);
+  q.t.hy = steps * R;
+  q.t.rows = H->many_ty + 2 * q.t.hy + sp::MANY_SR - 1;
+  q.t.cg = 1;
+  while (q.t.cg * sp::many_w(sizeof(T)) < q.t.tx + 2 * q.t.hx) q.t.cg *= 2;
+  for (int a = 0; a < 2; ++a) q.t.wall[a] = H->d.boundary[2 * a] != SP_PERIODIC;
+  for (int i = 0; i < 4; ++i) q.bv[i] = T(H->d.boundary_value[i]);
+  const int nty = (H->n[1] + H->many_ty - 1) / H->many_ty;
+  const cudaError_t e = H->many->launch(&q, dim3(unsigned(q.t.ntx * nty), unsigned(H->batch)),
+                                        many_smem(H, H->many_ty, steps), H->stream);
+  if (e != cudaSuccess) return cuda_fail(H, e, "many-step launch");
+  ++H->launches;
+  H->cur = dst;
+  return SP_OK;
+}
+int launch_many(sp_handle* H, int steps) {
+  return H->esz == 4 ? launch_many_t<float>(H, steps) : launch_many_t<double>(H, steps);
 }
 
 template <class T>
@@ -441,13 +501,13 @@ int setup_2d_t(sp_handle* H) {
 bool applicable(const sp_handle* H, int v) {
   const sp::KernelInfo& k = H->variants[v];
   if (k.kt > 1) {
-    // temporally blocked: 2D, periodic on both axes, x extents in whole copies
+    // temporally blocked: 2D, periodic on both axes
     if (H->dim != 2) return false;
     for (int s = 0; s < 4; ++s)
       if (H->d.boundary[s] != SP_PERIODIC) return false;
-    for (const InstGeo& g : H->geo)
-      if (g.n[0] % k.x_multiple != 0) return false;
   }
+  for (const InstGeo& g : H->geo)
+    if (g.n[0] % k.x_multiple != 0) return false;
   if (k.nx_only == 0) return true;
   if (H->dim != 3 || H->d.boundary[0] != SP_PERIODIC) return false;
   for (const InstGeo& g : H->geo)
@@ -547,6 +607,70 @@ int configure(sp_handle* H, int variant) {
     SP_CUDA(H, cudaMalloc(&H->partial_d, sizeof(double) * partial_n));
   }
   return SP_OK;
+}
+
+// Whether the many-step kernel takes this handle's steps, and its tile and
+// depth.  SP_MANY="tx,ty,kt" fixes them, SP_MANY=0 turns it off.
+void many_plan(sp_handle* H, const sp::ManyInfo* mi) {
+  H->many = nullptr;
+  if (!mi || H->dim != 2 || H->ensemble) return;
+  // (a 16-byte group of a narrower row would have images beyond both faces)
+  if (H->n[0] < 2 * sp::many_w(int(H->esz))) return;
+  const int n0 = H->n[0], n1 = H->n[1], R = mi->R;
+  const size_t row = size_t(mi->planes) * sp::MANY_PW * H->esz;
+  auto fits = [&](int tx, int ty, int kt) {
+    const int rows = ty + 2 * kt * R + sp::MANY_SR - 1;
+    return tx >= 4 && tx % 4 == 0 && ty >= 1 && kt >= 1 &&
+           tx + 2 * many_hx(H, kt, R) <= sp::MANY_PW && rows * row <= 227 * 1024 &&
+           (long long)((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty) * H->batch <= H->sms;
+  };
+  if (const char* e = getenv("SP_MANY")) {
+    int tx = 0, ty = 0, kt = 0;
+    if (sscanf(e, "%d,%d,%d", &tx, &ty, &kt) == 3 && fits(tx, ty, kt)) {
+      H->many = mi;
+      H->many_tx = tx;
+      H->many_ty = ty;
+      H->many_kt = kt;
+    }
+    return;
+  }
+  // Estimated microseconds, from timing every tile and depth on grids from 64^2
+  // to 804 x 601: a launch with its load costs 2.2, a sweep of the threads over
+  // a region (two rows of a column group each) 0.40, and 0.32 more when every
+  // thread has work; expressions that read a bilaplacian's points at each site
+  // cost three times that, a second field half as much again.  A step of the
+  // one-step kernels costs 3.0 and its sites.
+  const sp::KernelInfo& k = *H->ki;
+  const bool staged = k.ns > 0;
+  const double weight = (!staged && R > 1 ? 3.0 : 1.0) * (k.nf > 1 ? 1.5 : 1.0);
+  const double one = 3.0 + 1.4e-6 * n0 * n1 * H->batch * k.nf * double(H->esz / 4) * (staged ? 2.2 : 1.0);
+  double best = 0.85 * one;
+  for (int kt : {2, 4, 6, 8, 12, 16})
+    for (int gx = 1; gx * H->batch <= H->sms; ++gx) {
+      const int tx = ((n0 + gx - 1) / gx + 3) / 4 * 4, gy = H->sms / (gx * H->batch);
+      const int ty = (n1 + gy - 1) / gy;
+      if (!fits(tx, ty, kt)) continue;
+      int cg = 1;
+      while (cg * sp::many_w(int(H->esz)) < tx + 2 * many_hx(H, kt, R)) cg *= 2;
+      const int sweep = sp::MANY_NT / cg * sp::MANY_SR;  // rows of a sweep
+      double t = 2.2;
+      for (int j = 0; j < kt; ++j) {
+        const int rows = ty + 2 * (kt - 1 - j) * R;
+        const double w = double(tx + 2 * (kt - 1 - j) * R) / (cg * sp::many_w(int(H->esz)));
+        for (int phase = 0; phase < (staged ? 2 : 1); ++phase) {
+          const int n = (rows + 2 * phase + sweep - 1) / sweep;
+          t += weight * (0.40 * n + 0.32 * w * double(rows) / sweep);
+        }
+      }
+      t /= kt;
+      if (t < best * 0.999) {
+        best = t;
+        H->many = mi;
+        H->many_tx = tx;
+        H->many_ty = ty;
+        H->many_kt = kt;
+      }
+    }
 }
 
 // fastest tile shape of each (kernel key, extents, batch) found so far
@@ -689,6 +813,7 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   if (const char* t = getenv("SP_TILE")) variant = atoi(t);
   if (variant < 0 || variant >= int(H->variants.size()) || !applicable(H, variant)) variant = 0;
   if (int rc = configure(H, variant)) return rc;
+  if (!getenv("SP_TILE")) many_plan(H, sp::find_many(key));
   SP_CUDA(H, cudaDeviceSynchronize());
   return SP_OK;
 }
@@ -774,7 +899,8 @@ int capture_graph(sp_handle* H) {
   }
   int rc = SP_OK;
   const long long before = H->launches;
-  for (int i = 0; i < GRAPH_STEPS && rc == SP_OK; ++i) rc = launch_step(H, 0, nullptr, H->ki->kt);
+  for (int i = 0; i < GRAPH_STEPS && rc == SP_OK; ++i)
+    rc = H->many ? launch_many(H, H->many_kt) : launch_step(H, 0, nullptr, H->ki->kt);
   cudaError_t e = cudaStreamEndCapture(H->stream, &g);
   H->launches = before;
   H->cur = parity;
@@ -1017,18 +1143,27 @@ int sp_conserve_mass(sp_handle* H, int every) {
 namespace {
 int step_plain(sp_handle* H, int nsteps) {
   // a graph replays GRAPH_STEPS launches of kt steps each
-  const int kt = H->ki->kt, chunk = GRAPH_STEPS * kt;
+  const int kt = H->many ? H->many_kt : H->ki->kt, chunk = GRAPH_STEPS * kt;
+  // with the many-step kernel a single step (and the last one, where the state
+  // before it must stay in the other buffer) takes the one-step kernel
+  const int tail = H->many && H->keep_prev ? 1 : 0;
   while (nsteps > 0) {
-    if (nsteps >= chunk && H->graphs && !H->gexec[H->cur])
+    if (nsteps >= chunk + tail && H->graphs && !H->gexec[H->cur])
       if (int rc = capture_graph(H)) return rc;
-    if (nsteps >= chunk && H->gexec[H->cur]) {
+    if (nsteps >= chunk + tail && H->gexec[H->cur]) {
       SP_CUDA(H, cudaGraphLaunch(H->gexec[H->cur], H->stream));
       H->launches += GRAPH_STEPS;
       nsteps -= chunk;
-    } else {
-      const int s = std::min(kt, nsteps);
-      if (int rc = launch_step(H, 0, nullptr, s)) return rc;
+      continue;
+    }
+    const int s = std::min(kt, nsteps - tail);
+    if (H->many && s > 1) {
+      if (int rc = launch_many(H, s)) return rc;
       nsteps -= s;
+    } else {
+      const int s1 = H->many ? 1 : s;
+      if (int rc = launch_step(H, 0, nullptr, s1)) return rc;
+      nsteps -= s1;
     }
   }
   return SP_OK;
@@ -1085,6 +1220,8 @@ int sp_autotune(sp_handle* H, int reps) {
   if (!H || reps < 1) return SP_EINVAL;
   if (H->variants.size() < 2) return SP_OK;
   const long long launches = H->launches;
+  const sp::ManyInfo* const many = H->many;
+  H->many = nullptr;  // (put back below if it wins)
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   SP_CUDA(H, cudaEventCreate(&e0));
   SP_CUDA(H, cudaEventCreate(&e1));
@@ -1117,6 +1254,25 @@ int sp_autotune(sp_handle* H, int reps) {
       best = v;
     }
   }
+  if (rc == SP_OK && many) {
+    // many steps per launch: timed like the temporally blocked shapes
+    H->many = many;
+    const int cur = H->cur;
+    auto once = [&]() {
+      const int r = launch_many(H, H->many_kt);
+      H->cur = cur;
+      return r;
+    };
+    for (int i = 0; i < 2 && rc == SP_OK; ++i) rc = once();
+    cudaEventRecord(e0, H->stream);
+    for (int i = 0; i < reps && rc == SP_OK; ++i) rc = once();
+    cudaEventRecord(e1, H->stream);
+    if (rc == SP_OK && cudaEventSynchronize(e1) != cudaSuccess)
+      rc = fail(H, SP_ECUDA, "autotune timing failed");
+    float ms = 0.f;
+    if (rc == SP_OK) cudaEventElapsedTime(&ms, e0, e1);
+    if (ms / float(H->many_kt) >= best_ms) H->many = nullptr;
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   H->launches = launches;
@@ -1131,7 +1287,7 @@ int sp_autotune(sp_handle* H, int reps) {
 
 int sp_steps_per_launch(const sp_handle* H, int* kt) {
   if (!H || !kt) return SP_EINVAL;
-  *kt = H->ki->kt;
+  *kt = H->many ? H->many_kt : H->ki->kt;
   return SP_OK;
 }
 

@@ -67,6 +67,11 @@ struct sp_handle {
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   bool graphs = true;  // false once capture failed on this stream
   long long launches = 0;
+  // many steps per launch (2D grids of one wave of CTAs): the kernel and its
+  // tile, null where the grid or the key has none
+  const sp::ManyInfo* many = nullptr;
+  int many_tx = 0, many_ty = 0, many_kt = 0;
+  bool keep_prev = false;  // the other buffer must hold the state one step before
   // mass conservation of field 0 (sp_conserve_mass): every `conserve_every`
   // steps, restore each instance's mass to its target (2 doubles per instance:
   // the target mass and the energy reduced alongside it)

@@ -1,0 +1,22 @@
+/*
+ * sp_inst_many.cu -- many-step 2D kernels (sp_many2.cuh) of the FUSED form, for
+ * the keys of sp_inst_fused.cu.
+ */
+#include "sp_launch.cuh"
+
+#define SP_FUSED_MANY(T, DT)                                       \
+  SP_REGMANY(SPK_A, SPK_FUSED, MF_A_fused, T, DT, 5, 6, 13);       \
+  SP_REGMANY(SPK_B, SPK_FUSED, MF_B_fused, T, DT, 5, 6, 13);       \
+  SP_REGMANY(SPK_C, SPK_FUSED, MF_C_fused, T, DT, 5, 6, 13);       \
+  SP_REGMANY(SPK_AMK, SPK_FUSED, MF_AMK_fused, T, DT, 5, 6, 13);   \
+  SP_REGMANY(SPK_BMK, SPK_FUSED, MF_BMK_fused, T, DT, 5, 6, 13);   \
+  SP_REGMANY(SPK_A, SPK_FUSED, MF_A_fused, T, DT, 9, 6, 13);       \
+  SP_REGMANY(SPK_B, SPK_FUSED, MF_B_exact, T, DT, 9, 6, 13);       \
+  SP_REGMANY(SPK_C, SPK_FUSED, MF_C_exact, T, DT, 9, 6, 13);
+
+namespace sp {
+void register_many_kernels() {
+  SP_FUSED_MANY(float, 0)
+  SP_FUSED_MANY(double, 1)
+}
+}  // namespace sp

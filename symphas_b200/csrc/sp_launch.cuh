@@ -7,6 +7,7 @@
 #include "sp_chrow.cuh"
 #include "sp_row.cuh"
 #include "sp_kernels.cuh"
+#include "sp_many2.cuh"
 #include "sp_models.cuh"
 #include "sp_tb2.cuh"
 #include "sp_registry.h"
@@ -209,6 +210,22 @@ struct Entry2T {
   }
 };
 
+// many steps per launch (sp_many2.cuh)
+template <class MF, class T, int LP, int GP, int BP, bool EXACT>
+struct EntryMany {
+  using M = model_of<MF>;
+  using K = Fd2M<M, T, LP, GP, BP, EXACT>;
+  static cudaError_t launch(const void* prm, dim3 grid, size_t smem, cudaStream_t s) {
+    auto kern = k_fd2m<M, T, LP, GP, BP, EXACT>;
+    static cudaError_t attr = cudaFuncSetAttribute(
+        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (attr != cudaSuccess) return attr;
+    const M m = MF{}();
+    return launch_pdl(kern, grid, K::NT, smem, s, *static_cast<const ManyParams<T>*>(prm), m);
+  }
+  static ManyInfo info() { return ManyInfo{K::PLANES, K::R, &launch}; }
+};
+
 // model factories
 #define SP_FACTORY(NAME, EXPR)                          \
   struct NAME {                                         \
@@ -330,3 +347,6 @@ template <> struct Tiles<double> {
 #define SP_REG2X(MODEL, FORM, MF0, MF1, T, DT, LP, GP, BP)                 \
   ::sp::register_kernel(::sp::KernelKey{MODEL, FORM, 2, DT, LP, GP, BP},    \
                         ::sp::Entry2<::sp::MF0, ::sp::MF1, T, LP, GP, BP, ::sp::Tiles<T>::D2, FORM == SPK_EXACT>::info())
+#define SP_REGMANY(MODEL, FORM, MF, T, DT, LP, GP, BP)                       \
+  ::sp::register_many(::sp::KernelKey{MODEL, FORM, 2, DT, LP, GP, BP},        \
+                      ::sp::EntryMany<::sp::MF, T, LP, GP, BP, FORM == SPK_EXACT>::info())

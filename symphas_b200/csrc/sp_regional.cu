@@ -550,6 +550,7 @@ int make_window(sp_regional* R, const int o[3], const int d[3], sp_handle** out)
   }
   if (int rc = sp_create(&wd, out))
     return rfail(R, rc, std::string("window handle: ") + sp_create_error());
+  (*out)->keep_prev = true;  // rim images show the state before the last step
   if (R->stream)
     if (int rc = sp_set_stream(*out, R->stream)) {
       const std::string why = sp_last_error(*out);

@@ -44,11 +44,19 @@ struct KernelInfo {
   // nonzero: the kernel runs only on 3D grids of this x extent, periodic in x
   int nx_only = 0;
   // steps one launch can advance (temporally blocked kernels: > 1); such a
-  // kernel runs only on 2D grids periodic on both axes whose x extents are
-  // multiples of x_multiple
+  // kernel runs only on 2D grids periodic on both axes
   int kt = 1;
-  int x_multiple = 1;
+  int x_multiple = 1;  // every x extent must be a multiple of it
 };
+
+// the many-step kernel of a 2D key (sp_many2.cuh): `params` is ManyParams<T>
+struct ManyInfo {
+  int planes;  // shared-memory planes: two per field and one per staged operand
+  int R;       // reach of a step
+  cudaError_t (*launch)(const void* params, dim3 grid, size_t smem, cudaStream_t s);
+};
+void register_many(const KernelKey& key, const ManyInfo& info);
+const ManyInfo* find_many(const KernelKey& key);
 
 // appends a tile variant for `key` (the first registered is the default)
 void register_kernel(const KernelKey& key, const KernelInfo& info);

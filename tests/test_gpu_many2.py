@@ -1,0 +1,77 @@
+"""Many steps per launch on small 2D grids (sp_many2.cuh): every step count
+gives the bits of the one-step tile kernel, on ragged and tiny grids, with
+periodic, constant and mixed sides (different constants on each), batches, both
+dtypes and forms, all models; the many-step kernel at chosen tiles and depths
+(tiles that do not divide the grid, depths past the grid's own extent), the
+state before the last step for moving windows' rims, and mass conservation."""
+import numpy as np
+import pytest
+
+import symphas_b200 as sp
+
+pytestmark = pytest.mark.gpu
+
+P, D = sp.BoundaryType.PERIODIC, sp.BoundaryType.DEFAULT
+MODELS = {"A": sp.model_MA_t, "B": sp.model_MB_t, "C": sp.model_MC_t, "AMK": sp.model_MAMK_t,
+          "BMK": sp.model_MBMK_t}
+WALLS = {"": [P] * 6, "x": [D, D, P, P, P, P], "y": [P, P, D, D, P, P], "xy": [D, D, D, D, P, P]}
+
+
+def run(monkeypatch, env, model, dims, dtype, form, steps, walls="", batch=1, wide=False, chunks=(),
+        conserve=0):
+    for k in ("SP_TILE", "SP_MANY"):
+        monkeypatch.delenv(k, raising=False)
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    st = sp.Stencil2d2h() if wide else sp.Stencil2d2h(5, 6, 13)
+    params = sp.ProblemParameters(dims, boundary=WALLS[walls],
+                                  boundary_value=[0.3, -0.2, 0.15, 0.05, 0.0, 0.0])
+    m = MODELS[model](2, sp.SolverFT(st, form=form), params, coeff=(0.8, 1.1), dtype=dtype,
+                      batch=batch)
+    for i in range(batch):
+        for f in range(m.nfields):
+            m.fill_uniform(f, 31 + 7 * i + f, -0.3, 0.2, inst=i)
+    if conserve:
+        m.conserve_mass(conserve)
+    for s in chunks or (steps,):
+        m.step(0.01, s)
+    out = np.stack([m.get_field(f, inst=i) for i in range(batch) for f in range(m.nfields)])
+    info, launches = m.kernel_info(), m.launch_count()
+    m.close()
+    return out, info, launches
+
+
+@pytest.mark.parametrize("model,dtype,form", [("A", "f64", "exact"), ("B", "f32", "fused"),
+                                              ("B", "f64", "exact"), ("C", "f32", "fused"),
+                                              ("C", "f64", "exact"), ("AMK", "f32", "fused"),
+                                              ("BMK", "f64", "fused")])
+@pytest.mark.parametrize("dims,many", [((64, 64), "16,8,8"), ((37, 21), "12,5,4"),
+                                       ((9, 130), "8,40,3"), ((101, 53), "40,16,6")])
+@pytest.mark.parametrize("walls", ["", "x", "y", "xy"])
+def test_many_steps_match_single_steps(model, dtype, form, dims, many, walls, monkeypatch):
+    want, info, n1 = run(monkeypatch, {"SP_MANY": "0"}, model, dims, dtype, form, 19, walls)
+    assert info["steps_per_launch"] == 1 and n1 == 19
+    got, info, n = run(monkeypatch, {"SP_MANY": many}, model, dims, dtype, form, 19, walls)
+    assert info["steps_per_launch"] == int(many.split(",")[2]) and n < n1
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("dims,kw", [((64, 64), {}), ((16, 12), {}), ((300, 200), {"batch": 3}),
+                                     ((255, 129), {"wide": True}), ((804, 601), {}),
+                                     ((48, 48), {"conserve": 7}), ((70, 50), {"walls": "xy"})])
+@pytest.mark.parametrize("model,dtype,form", [("A", "f32", "fused"), ("B", "f32", "fused"),
+                                              ("B", "f64", "exact")])
+def test_chosen_depth_matches_single_steps(model, dtype, form, dims, kw, monkeypatch):
+    """The depth the library chooses, over calls of different lengths (graph
+    replay, remainders, single steps)."""
+    chunks = (1, 2, 600, 33, 5)
+    want, _, _ = run(monkeypatch, {"SP_MANY": "0"}, model, dims, dtype, form, 0, chunks=chunks, **kw)
+    got, info, _ = run(monkeypatch, {}, model, dims, dtype, form, 0, chunks=chunks, **kw)
+    if dims == (64, 64):
+        assert info["steps_per_launch"] > 1
+    if kw.get("wide") and form == "fused":
+        # the term order of the exact form compiled with contraction: which
+        # products fuse is the compiler's choice per kernel, one rounding each
+        assert np.abs(got - want).max() <= 641 * 2.0 ** -24
+    else:
+        assert np.array_equal(got, want)
