@@ -222,6 +222,7 @@ int launch_step_t(sp_handle* H, int rhs_only, double* partial, int steps, bool a
     p.err = H->err_d;
     p.in = reinterpret_cast<const T* const*>(H->outs_d[src]);
     p.tsteps = steps;
+    p.ty = H->ki->ty;
     e = H->ki->launch(&p, dim3(H->grid2), H->stream);
   }
   if (e != cudaSuccess) return cuda_fail(H, e, "fused step launch");
@@ -492,8 +493,24 @@ int setup_2d_t(sp_handle* H) {
     SP_CUDA(H, cudaMemset(H->ctr_d, 0, 2 * sizeof(int)));
   }
   const int occ = H->ki->occupancy();
-  H->grid2 = std::max(1, std::min(H->sms * occ, H->nitems));
+  H->grid2 = H->ki->item_warps ? (H->nitems + H->ki->item_warps - 1) / H->ki->item_warps
+                               : std::max(1, std::min(H->sms * occ, H->nitems));
   return SP_OK;
+}
+
+// Rows of a warp-strip item: an item reads up to four rows more than it
+// writes, so long items read less and short ones fill the SMs.  Two waves of
+// the resident warps, between 8 and 16 rows (timed from 64^2 x 1024 to 4096^2:
+// 12 to 16 are within 3 % of the best there, 32 and more up to 40 % slower), 24
+// on grids of a hundred waves.  SP_STRIP_ROWS fixes it.
+int strip_rows(const sp_handle* H, const sp::KernelInfo& k) {
+  if (const char* e = getenv("SP_STRIP_ROWS"))
+    if (atoi(e) > 0) return std::min(atoi(e), 200);
+  long long rows = 0;
+  for (const InstGeo& g : H->geo) rows += (long long)((g.n[0] + k.tx - 1) / k.tx) * g.n[1];
+  const long long slots = (long long)H->sms * k.occupancy() * k.item_warps;
+  const long long t = rows / (2 * slots);
+  return t >= 96 ? 24 : int(std::min(16LL, std::max(8LL, t)));
 }
 
 // whether tile variant v can run this handle's grid (row kernels need every
@@ -507,7 +524,7 @@ bool applicable(const sp_handle* H, int v) {
       if (H->d.boundary[s] != SP_PERIODIC) return false;
   }
   for (const InstGeo& g : H->geo)
-    if (g.n[0] % k.x_multiple != 0) return false;
+    if (g.n[0] % k.x_multiple != 0 || g.n[0] < k.x_min) return false;
   if (k.nx_only == 0) return true;
   if (H->dim != 3 || H->d.boundary[0] != SP_PERIODIC) return false;
   for (const InstGeo& g : H->geo)
@@ -521,6 +538,8 @@ bool applicable(const sp_handle* H, int v) {
 int configure(sp_handle* H, int variant) {
   SP_CUDA(H, cudaStreamSynchronize(H->stream));
   H->variant = variant;
+  if (H->variants[variant].item_warps)
+    H->variants[variant].ty = strip_rows(H, H->variants[variant]);
   H->ki = &H->variants[variant];
   const int R = H->ki->R;
   H->ntx = (H->n[0] + H->ki->tx - 1) / H->ki->tx;
@@ -805,6 +824,8 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   // tile shape: an explicit choice (SP_TILE), else the one sp_autotune found
   // for this kernel and size in this process, else the first registered
   int variant = 0;
+  for (int v = 1; v < int(H->variants.size()); ++v)
+    if (H->variants[v].pref > H->variants[variant].pref && applicable(H, v)) variant = v;
   if (!H->ensemble) {
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     auto it = g_tuned.find(tune_key(H));

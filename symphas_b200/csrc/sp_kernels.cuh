@@ -84,6 +84,7 @@ struct Step2Params {
   // [inst * nf + f], and the steps of this launch (1 .. the kernel's KT)
   const T* const* in;
   int tsteps;
+  int ty;  // rows of an item (sp_strip2.cuh)
 };
 
 // ---------------------------------------------------------------------------

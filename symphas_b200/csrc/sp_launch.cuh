@@ -9,6 +9,7 @@
 #include "sp_kernels.cuh"
 #include "sp_many2.cuh"
 #include "sp_models.cuh"
+#include "sp_strip2.cuh"
 #include "sp_tb2.cuh"
 #include "sp_registry.h"
 
@@ -210,6 +211,38 @@ struct Entry2T {
   }
 };
 
+// the warp-strip 2D step (sp_strip2.cuh)
+template <class MF0, class MF1, int PF, int PREF>
+struct EntryStrip2 {
+  using M0 = model_of<MF0>;
+  using M1 = model_of<MF1>;
+  static constexpr int R = imax(M0::R, M1::R), RS = imax(M0::ns ? M0::RS : 0, M1::ns ? M1::RS : 0),
+                       NS = imax(M0::ns, M1::ns), RI = imax(imax(M0::r_stage, M1::r_stage), 0);
+  static constexpr int HXA = HaloGeom<float, 4, R, NS, RS, RI>::HXA;
+  static_assert(HXA >= 4, "a lane left of the strip lies in the halo");
+  static cudaError_t launch(const void* prm, dim3 grid, cudaStream_t s) {
+    const M0 m0 = MF0{}();
+    const M1 m1 = MF1{}();
+    return launch_pdl(k_fd2w<M0, M1, PF>, grid, 32 * ST2_WARPS, 0, s,
+                      *static_cast<const Step2Params<float>*>(prm), m0, m1);
+  }
+  static int occupancy() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fd2w<M0, M1, PF>, 32 * ST2_WARPS, 0) !=
+        cudaSuccess)
+      return 1;
+    return n > 0 ? n : 1;
+  }
+  static KernelInfo info() {
+    KernelInfo i{M0::nf, NS, R, HXA, ST2_X, 32, 1, PF, 32 * ST2_WARPS, 0, &launch, &occupancy};
+    i.item_warps = ST2_WARPS;
+    i.x_multiple = 4;
+    i.x_min = 8;  // a lane's group has periodic images beyond one face at most
+    i.pref = PREF;
+    return i;
+  }
+};
+
 // many steps per launch (sp_many2.cuh)
 template <class MF, class T, int LP, int GP, int BP, bool EXACT>
 struct EntryMany {
@@ -350,3 +383,6 @@ template <> struct Tiles<double> {
 #define SP_REGMANY(MODEL, FORM, MF, T, DT, LP, GP, BP)                       \
   ::sp::register_many(::sp::KernelKey{MODEL, FORM, 2, DT, LP, GP, BP},        \
                       ::sp::EntryMany<::sp::MF, T, LP, GP, BP, FORM == SPK_EXACT>::info())
+#define SP_REGSTRIP2(MODEL, MF0, MF1, PF, PREF)                              \
+  ::sp::register_kernel(::sp::KernelKey{MODEL, SPK_FUSED, 2, 0, 5, 6, 13},    \
+                        ::sp::EntryStrip2<::sp::MF0, ::sp::MF1, PF, PREF>::info())

@@ -47,6 +47,12 @@ struct KernelInfo {
   // kernel runs only on 2D grids periodic on both axes
   int kt = 1;
   int x_multiple = 1;  // every x extent must be a multiple of it
+  int x_min = 0;       // and at least this
+  // 2D kernels whose items are taken one per warp, this many warps per CTA (0:
+  // CTAs take tiles); ty is then chosen for the grid
+  int item_warps = 0;
+  // sp_create starts with the applicable variant of the highest preference
+  int pref = 0;
 };
 
 // the many-step kernel of a 2D key (sp_many2.cuh): `params` is ManyParams<T>

@@ -1,7 +1,8 @@
-"""Many steps per launch on small 2D grids (sp_many2.cuh): every step count
-gives the bits of the one-step tile kernel, on ragged and tiny grids, with
-periodic, constant and mixed sides (different constants on each), batches, both
-dtypes and forms, all models; the many-step kernel at chosen tiles and depths
+"""Many steps per launch on small 2D grids (sp_many2.cuh) and the warp-strip 2D
+step (sp_strip2.cuh): every step count and shape gives the bits of the one-step
+tile kernel, on ragged and tiny grids, with periodic, constant and mixed sides
+(different constants on each), batches, both dtypes and forms, all models, and
+for ensembles of mixed members; the many-step kernel at chosen tiles and depths
 (tiles that do not divide the grid, depths past the grid's own extent), the
 state before the last step for moving windows' rims, and mass conservation."""
 import numpy as np
@@ -75,3 +76,52 @@ def test_chosen_depth_matches_single_steps(model, dtype, form, dims, kw, monkeyp
         assert np.abs(got - want).max() <= 641 * 2.0 ** -24
     else:
         assert np.array_equal(got, want)
+
+
+def strip_variants(monkeypatch, model, dims):
+    _, info, _ = run(monkeypatch, {"SP_TILE": "0"}, model, dims, "f32", "fused", 1)
+    out = []
+    for v in range(info["variants"]):
+        _, i, _ = run(monkeypatch, {"SP_TILE": str(v)}, model, dims, "f32", "fused", 1)
+        if i["variant"] == v and i["tile_x"] == 120:
+            out.append(v)
+    return out
+
+
+@pytest.mark.parametrize("model", sorted(MODELS))
+@pytest.mark.parametrize("dims", [(8, 9), (120, 40), (124, 33), (256, 64), (480, 17), (1000, 70)])
+@pytest.mark.parametrize("walls", ["", "x", "xy"])
+def test_strip_step_matches_tile_step(model, dims, walls, monkeypatch):
+    vs = strip_variants(monkeypatch, model, (128, 64))
+    assert vs
+    want, _, _ = run(monkeypatch, {"SP_TILE": "0"}, model, dims, "f32", "fused", 9, walls, batch=2)
+    for v in vs:
+        got, info, _ = run(monkeypatch, {"SP_TILE": str(v)}, model, dims, "f32", "fused", 9, walls,
+                           batch=2)
+        assert info["variant"] == v
+        assert np.array_equal(got, want)
+    # ragged rows, and rows a group of which lies at both faces, keep the tile kernel
+    for d in ((130, 40), (4, 40)):
+        _, info, _ = run(monkeypatch, {"SP_TILE": str(vs[0])}, model, d, "f32", "fused", 1)
+        assert info["variant"] == 0
+
+
+def test_strip_step_on_ensembles(monkeypatch):
+    members = sp.ensemble_members(12, seed=3, sides=(64, 96, 128, 256, 384))
+    outs = {}
+    e = sp.Ensemble(sp.SolverFT(sp.Stencil2d2h(5, 6, 13)), members)
+    nv = e.kernel_info()["variants"]
+    e.close()
+    for v in range(nv):
+        monkeypatch.setenv("SP_TILE", str(v))
+        e = sp.Ensemble(sp.SolverFT(sp.Stencil2d2h(5, 6, 13)), members)
+        if e.kernel_info()["variant"] == v and (v == 0 or e.kernel_info()["tile_x"] == 120):
+            for i in range(len(members)):
+                e.fill_uniform(0, 5 + i, -0.1, 0.1, inst=i)
+            e.step(41)
+            outs[v] = [e.get_field(0, inst=i) for i in range(len(members))]
+        e.close()
+    assert len(outs) > 1
+    for v in outs:
+        for a, b in zip(outs[0], outs[v]):
+            assert np.array_equal(a, b), v
