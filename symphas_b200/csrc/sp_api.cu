@@ -64,6 +64,7 @@ const ManyInfo* find_many(const KernelKey& key) {
 void register_exact_kernels() __attribute__((weak));
 void register_fused_kernels() __attribute__((weak));
 void register_wide_kernels() __attribute__((weak));
+void register_exact3_kernels() __attribute__((weak));
 void register_many_kernels() __attribute__((weak));
 void register_many_exact_kernels() __attribute__((weak));
 void register_all_kernels() {
@@ -72,6 +73,7 @@ void register_all_kernels() {
     if (register_exact_kernels) register_exact_kernels();
     if (register_fused_kernels) register_fused_kernels();
     if (register_wide_kernels) register_wide_kernels();
+    if (register_exact3_kernels) register_exact3_kernels();
     if (register_many_kernels) register_many_kernels();
     if (register_many_exact_kernels) register_many_exact_kernels();
   });

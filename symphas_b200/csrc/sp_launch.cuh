@@ -349,6 +349,9 @@ template <> struct Tiles<float> {
 template <> struct Tiles<double> {
   using D3 = TileCfg<64, 16, 2, 3, 2>;
   using D2 = TileCfg<64, 16, 4, 3, 2>;
+  using D3b = TileCfg<64, 16, 4, 2, 2>;
+  using D3c = TileCfg<64, 8, 4, 2, 2>;
+  using D3d = TileCfg<32, 16, 4, 2, 2>;
   using T2a = TbCfg<64, 32, 2, 256, 2>;
 };
 }  // namespace sp
