@@ -608,7 +608,13 @@ int configure(sp_handle* H, int variant) {
     const long long tiles = (long long)H->ntx * H->nty * H->batch;
     const long long slots = (long long)H->sms * occ;
     int chunks = int(std::max(1LL, slots / tiles));
-    chunks = std::min(chunks, std::max(1, H->n[2] / std::max(4, 2 * R)));
+    // Chunks of at least 4 planes (each reads 2R planes more than it writes),
+    // but down to one plane while that gives an SM no more than two CTAs: a
+    // plane costs a CTA about 1 us of latency whatever its work, so a grid of a
+    // few tiles is bound by the length of its march (64^3, us with 4 planes and
+    // with 1: A 5.4 and 3.0, B 7.4 and 4.5, C 9.6 and 5.6).
+    const long long most = std::max<long long>(H->n[2] / std::max(4, 2 * R), 2LL * H->sms / tiles);
+    chunks = int(std::min<long long>(chunks, std::max(1LL, std::min<long long>(most, H->n[2]))));
     H->zchunk = (H->n[2] + chunks - 1) / chunks;
     if (const char* zc = getenv("SP_ZCHUNK")) {
       const int v = atoi(zc);
@@ -826,8 +832,15 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   // tile shape: an explicit choice (SP_TILE), else the one sp_autotune found
   // for this kernel and size in this process, else the first registered
   int variant = 0;
-  for (int v = 1; v < int(H->variants.size()); ++v)
-    if (H->variants[v].pref > H->variants[variant].pref && applicable(H, v)) variant = v;
+  long long sites = 0;
+  for (const InstGeo& g : H->geo) sites += g.sites();
+  for (int v = 1; v < int(H->variants.size()); ++v) {
+    const sp::KernelInfo& k = H->variants[v];
+    const double filled = H->n[0] / (64.0 * ((H->n[0] + 63) / 64));
+    if (k.pref > H->variants[variant].pref && H->n[0] % k.pref_x == 0 && H->n[0] >= k.pref_xmin &&
+        sites >= k.pref_sites && filled <= k.pref_filled && applicable(H, v))
+      variant = v;
+  }
   if (!H->ensemble) {
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     auto it = g_tuned.find(tune_key(H));

@@ -61,6 +61,13 @@ void register_fused_kernels() {
   SP_FUSED_VARIANTS3(SPK_A, MF_A_fused)
   SP_FUSED_VARIANTS3(SPK_B, MF_B_fused)
   SP_FUSED_VARIANTS3(SPK_C, MF_C_fused)
+  {
+    // model C starts with two rows a thread on any grid (64^3 5.5 -> 5.2 us,
+    // 98 x 33 x 210 13.3 -> 11.7, 150 x 131 x 97 22.0 -> 18.5)
+    KernelInfo i = Entry3<MF_C_fused, float, 7, 10, 25, Tiles<float>::D3e, false>::info();
+    i.pref = 1;
+    register_kernel(KernelKey{SPK_C, SPK_FUSED, 3, 0, 7, 10, 25}, i);
+  }
   SP_FUSED_VARIANTS2(SPK_A, MF_A_fused, MF_A_fused)
   SP_FUSED_VARIANTS2(SPK_B, MF_B_fused, MF_B_fused)
   SP_FUSED_VARIANTS2(SPK_ENS_AB, MF_AMK_fused, MF_BMK_fused)

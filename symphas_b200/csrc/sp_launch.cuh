@@ -334,6 +334,8 @@ template <> struct Tiles<float> {
   using D3w3 = TileCfg<64, 16, 2, 2, 4>;
   using D3w4 = TileCfg<128, 16, 2, 2, 4>;
   using D3w5 = TileCfg<64, 32, 4, 2, 4>;
+  using D3n1 = TileCfg<32, 16, 2, 2, 2>;  // narrow tiles for extents 64 does not fill
+  using D3n2 = TileCfg<32, 16, 4, 3, 2>;
   using D2w1 = TileCfg<128, 16, 4, 3, 4>;
   using D2w2 = TileCfg<128, 32, 4, 2, 4>;
   using D2w3 = TileCfg<128, 16, 2, 3, 4>;

@@ -52,7 +52,13 @@ struct KernelInfo {
   // CTAs take tiles); ty is then chosen for the grid
   int item_warps = 0;
   // sp_create starts with the applicable variant of the highest preference
+  // whose conditions hold: an x extent that is a multiple of pref_x, at least
+  // pref_xmin and fills its 64-wide tiles to at most pref_filled, and
+  // pref_sites sites in all
   int pref = 0;
+  int pref_x = 1, pref_xmin = 0;
+  double pref_filled = 1.0;
+  long long pref_sites = 0;
 };
 
 // the many-step kernel of a 2D key (sp_many2.cuh): `params` is ManyParams<T>
