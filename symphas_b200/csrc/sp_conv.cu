@@ -1094,26 +1094,31 @@ int launch_strip(StripParams p, int* err, cudaStream_t s, int smax) {
 #include "sp_flow.cuh"
 
 namespace {
-// the persistent kernel (sp_flow.cuh) where it can run: input channels in
-// whole stages, and shared memory for the weights and two strips; SP_EINVAL
-// otherwise
-int flow_fwd(const sp::conv::FlowParams& p, int* err, cudaStream_t s) {
+// the persistent kernel (sp_flow.cuh) where it can run, SP_EINVAL otherwise: the
+// largest tile that leaves room for two strips (a strip's reach beyond its tile,
+// two rows, is gathered again by the next tile), with the weights resident, or
+// streamed from `wt` where they do not fit
+int flow_fwd(sp::conv::FlowParams p, void* wt, int* err, cudaStream_t s) {
   using namespace sp::conv;
-  if (p.cin % FL_CB != 0) return SP_EINVAL;
-  int P;
-  auto fits = [&](int MT, int BN) { return flow_stages(MT * 128, BN, p.cin, p.wid, &P) >= 2; };
-  // the largest tile that leaves room for two strips: a strip's reach beyond
-  // its tile (two rows) is gathered again by the next tile
+  int rc = SP_EINVAL;
   if (p.cout == 32) {
-    if (fits(8, 32)) return launch_flow<32, 8>(p, err, s);
-    if (fits(4, 32)) return launch_flow<32, 4>(p, err, s);
+    rc = launch_flow<32, 8>(p, err, s);
+    if (rc == SP_EINVAL) rc = launch_flow<32, 4>(p, err, s);
   } else if (p.cout == 64) {
-    if (fits(4, 64)) return launch_flow<64, 4>(p, err, s);
-    if (fits(2, 64)) return launch_flow<64, 2>(p, err, s);
+    rc = launch_flow<64, 4>(p, err, s);
+    if (rc == SP_EINVAL) rc = launch_flow<64, 2>(p, err, s);
   } else if (p.cout % 128 == 0) {
-    if (fits(2, 128)) return launch_flow<128, 2>(p, err, s);
+    rc = launch_flow<128, 2>(p, err, s);
+    int P;
+    if (rc == SP_EINVAL && p.cin % FL_CBS == 0 && flow_stages<128, 4, true>(p.cin, p.wid, &P)) {
+      k_tile_weights<<<256, 256, 0, s>>>(p.w, static_cast<__nv_bfloat16*>(wt), p.cin, p.cout, 128,
+                                          FL_CBS);
+      if (cudaGetLastError() != cudaSuccess) return SP_ECUDA;
+      p.w = static_cast<const __nv_bfloat16*>(wt);
+      rc = launch_flow<128, 4, true>(p, err, s);
+    }
   }
-  return SP_EINVAL;
+  return rc;
 }
 
 int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const void* res, void* z,
@@ -1139,7 +1144,7 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
                  static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(z),
                  static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout, 0, 0, 0, up,
                  al(res) && al(z) && al(a)};
-    const int rc = flow_fwd(f, err, s);
+    const int rc = flow_fwd(f, wt, err, s);
     if (rc != SP_EINVAL) return rc;
   }
   const int bn = cout == 32 ? 32 : cout == 64 ? 64 : 128;

@@ -27,13 +27,14 @@ namespace conv {
 
 constexpr int FL_PROD = 256, FL_EPI = 512;       // producer and epilogue threads
 constexpr int FL_NT = FL_PROD + 32 + FL_EPI;     // and the MMA warp
-constexpr int FL_CB = 32, FL_CH = FL_CB / 8;     // input channels per stage
+constexpr int FL_CB = 32;                        // input channels per stage, weights resident
+constexpr int FL_CBS = 16;                       // and streamed
 constexpr int FL_SMEM = 227 * 1024 - 1024;       // for weights and strips
 constexpr int FL_SMAX = 4;                       // stages of the ring
 
 struct FlowParams {
   const __nv_bfloat16* x;    // [N][H][W][Cin]
-  const __nv_bfloat16* w;    // [Cout][3][3][Cin]
+  const __nv_bfloat16* w;    // [Cout][3][3][Cin]; streamed: as k_tile_weights leaves them
   const float* bias;         // [Cout] or null
   const __nv_bfloat16* res;  // [N][H][W][Cout] or null
   __nv_bfloat16* z;          // pre-activation out, or null
@@ -149,28 +150,37 @@ struct PadPos {
   }
 };
 
-template <int BN, int MT>
+// STREAM: the weights do not fit beside the strips (128 outputs of 128 and more
+// inputs: 295 KB) and come with every stage, 16 input channels' share in one
+// bulk copy; then a tile is as large as tensor memory allows (MT = 4: one
+// accumulator set), so that a stage's 37 KB serve 512 positions, and the next
+// tile's first MMAs start as soon as the epilogue has emptied their block.
+template <int BN, int MT, bool STREAM>
 struct FlowTile {
   static constexpr int M = MT * 128;   // positions per tile
-  static constexpr int ACC = MT * BN;  // tensor-memory columns of one accumulator
-  static_assert(2 * ACC <= 512 && (2 * ACC & (2 * ACC - 1)) == 0 && 2 * ACC >= 32, "columns");
-  static_assert(BN % 32 == 0 && BN <= 128 && MT % 2 == 0, "tile");
+  static constexpr int ACC = MT * BN;  // tensor-memory columns of one accumulator set
+  static constexpr int NBUF = 2 * ACC <= 512 ? 2 : 1, COLS = NBUF * ACC;
+  static constexpr int CB = STREAM ? FL_CBS : FL_CB, CH = CB / 8;
+  static constexpr int WSTAGE = STREAM ? BN * 9 * CB * 2 : 0;  // bytes of a stage's weights
+  static constexpr int EWARPS = 4 * (BN / 32 < 4 ? BN / 32 : 4);  // warps that empty a block
+  static_assert(COLS <= 512 && (COLS & (COLS - 1)) == 0 && COLS >= 32, "columns");
+  static_assert(BN % 32 == 0 && BN <= 128 && MT % 2 == 0 && MT <= 8, "tile");
 };
 
-template <int BN, int MT>
+template <int BN, int MT, bool STREAM>
 __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, int* err) {
-  using TT = FlowTile<BN, MT>;
-  constexpr int M = TT::M, ACC = TT::ACC;
+  using TT = FlowTile<BN, MT, STREAM>;
+  constexpr int M = TT::M, ACC = TT::ACC, NBUF = TT::NBUF, CB = TT::CB, CH = TT::CH;
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int S = p.S, P = p.P, STAGE = FL_CH * P * 16;
+  const int S = p.S, P = p.P, STAGE = CH * P * 16 + TT::WSTAGE;
   const int kch = p.cin / 8;  // 8-channel chunks of the input
-  const int nkb = p.cin / FL_CB;
+  const int nkb = p.cin / CB;
   unsigned char* const wsm = smem;  // [9 * kch chunks][BN rows][16 B]
-  unsigned char* const ring = smem + 9 * kch * BN * 16;
+  unsigned char* const ring = smem + (STREAM ? 0 : 9 * kch * BN * 16);
   float* const bsm = reinterpret_cast<float*>(ring + S * STAGE);  // [BN] bias
   uint64_t* const bars = reinterpret_cast<uint64_t*>(bsm + BN);
   uint64_t *const full = bars, *const empty = bars + FL_SMAX, *const tfull = bars + 2 * FL_SMAX,
-           *const tempty = tfull + 2, *const done = tempty + 2;
+           *const tempty = tfull + 2, *const done = tempty + 2 * 8;
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int W2 = p.wid + 2, H2 = p.h + 2;
@@ -181,26 +191,27 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(2 * ACC));
+                 "r"(TT::COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      tma::mbar_init(&full[s], FL_PROD / 32);
+      tma::mbar_init(&full[s], FL_PROD / 32 + (STREAM ? 1 : 0));
       tma::mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < NBUF; ++b) {
       tma::mbar_init(&tfull[b], 1);
-      tma::mbar_init(&tempty[b], FL_EPI / 32);
+      for (int m = 0; m < MT; ++m) tma::mbar_init(&tempty[b * MT + m], TT::EWARPS);
     }
     tma::mbar_init(done, 1);
     tma::fence_barrier_init();
   }
   // the weights, K-major without swizzle: [tap * kch + chunk][output channel]
-  for (int i = tid; i < 9 * kch * BN; i += FL_NT) {
-    const int co = i % BN, kc = i / BN;
-    cp_async16(wsm + i * 16, p.w + ((long long)(co0 + co) * 9 * kch + kc) * 8, true);
-  }
+  if constexpr (!STREAM)
+    for (int i = tid; i < 9 * kch * BN; i += FL_NT) {
+      const int co = i % BN, kc = i / BN;
+      cp_async16(wsm + i * 16, p.w + ((long long)(co0 + co) * 9 * kch + kc) * 8, true);
+    }
   for (int i = tid; i < BN; i += FL_NT) bsm[i] = p.bias ? p.bias[co0 + i] : 0.f;
   asm volatile("cp.async.wait_all;" ::: "memory");
   tma::fence_proxy_async();  // generic-proxy writes, read by the tensor core
@@ -211,10 +222,10 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
   bool bad = false;
 
   if (warp < MMA_WARP) {
-    // ---- producers: a warp copies 8 positions x 4 chunks at a time; lane:
-    // position lp, chunk j
-    const int j = lane >> 3, lp = warp * 8 + (lane & 7);
-    constexpr int STEP = FL_PROD / FL_CH;
+    // ---- producers: a warp copies 32 / CH positions x CH chunks at a time;
+    // lane: position lp, chunk j
+    constexpr int LP = 32 / CH, STEP = FL_PROD / CH;
+    const int j = lane / LP, lp = warp * LP + lane % LP;
     const int sy = STEP / W2, sx = STEP - sy * W2;
     int s = 0;
     uint32_t ph = 1;  // a fresh barrier passes the wait for the phase before its first
@@ -230,7 +241,13 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
           break;
         }
         unsigned char* dst = ring + s * STAGE + (j * P + lp) * 16;
-        const __nv_bfloat16* const xc = p.x + kb * FL_CB + j * 8;
+        const __nv_bfloat16* const xc = p.x + kb * CB + j * 8;
+        if (STREAM && tid == 0) {
+          tma::mbar_arrive_expect_tx(&full[s], uint32_t(TT::WSTAGE));
+          bulk_load(ring + s * STAGE + CH * P * 16,
+                    p.w + (long long)(blockIdx.y * nkb + kb) * (TT::WSTAGE / 2),
+                    uint32_t(TT::WSTAGE), &full[s]);
+        }
         PadPos q = start;
 #pragma unroll 4
         for (int pos = lp; pos < P; pos += STEP) {
@@ -260,18 +277,17 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
       // ---- MMA issuer: per stage, for every tap and K step of 16 channels,
       // one MMA per 128 positions
       constexpr uint32_t idesc = umma_idesc<BN>();
-      constexpr uint32_t HI = (128u >> 4) | (1u << 14);  // 128 B between 8-row groups, version 1
-      const uint32_t alo = uint32_t(P) << 16, blo = uint32_t(BN) << 16;  // chunk strides / 16
+      // strips: 128 B between 8-row groups (SBO), P x 16 B between chunks (LBO);
+      // weights likewise with BN x 16 B, or as k_tile_weights lays them out
+      constexpr uint32_t AHI = (128u >> 4) | (1u << 14);
+      constexpr uint32_t BHI = (STREAM ? uint32_t(9 * CH * 8) : 128u >> 4) | (1u << 14);
+      const uint32_t alo = uint32_t(P) << 16, blo = (STREAM ? 8u : uint32_t(BN)) << 16;
       const uint32_t w0 = blo + (smem_u32(wsm) >> 4), r0 = alo + (smem_u32(ring) >> 4);
       int s = 0, it = 0;
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < p.tiles && !bad; tile += gridDim.x, ++it) {
-        const int b = it & 1;
-        if (!tma::mbar_wait(&tempty[b], uint32_t((it >> 1) & 1) ^ 1u)) {
-          bad = true;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int b = it % NBUF;
+        const uint32_t eph = uint32_t((it / NBUF) & 1) ^ 1u;
         const uint32_t acc = tmem + uint32_t(b * ACC);
         for (int kb = 0; kb < nkb; ++kb) {
           if (!tma::mbar_wait(&full[s], ph)) {
@@ -279,30 +295,55 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = r0 + uint32_t(s * FL_CH * P);
-          const uint32_t b0 = w0 + uint32_t(kb * FL_CH * BN);
-          auto tap = [&](int t, auto first) {
-            const uint32_t at = a0 + uint32_t((t / 3) * W2 + t % 3);  // position 0 of the tap
-            const uint32_t bt = b0 + uint32_t(t * kch * BN);
-#pragma unroll
-            for (int kk = 0; kk < FL_CB / 16; ++kk) {
-              const uint64_t bd = desc_at(bt + 2 * kk * BN, HI);
-              const uint32_t ak = at + uint32_t(2 * kk * P);
-#pragma unroll
-              for (int m = 0; m < MT; ++m) {
-                if (decltype(first)::value && kk == 0)
-                  umma_go<false>(acc + uint32_t(m * BN), desc_at(ak + m * 128, HI), bd, idesc);
-                else
-                  umma_go<true>(acc + uint32_t(m * BN), desc_at(ak + m * 128, HI), bd, idesc);
-              }
-            }
+          const uint32_t a0 = r0 + uint32_t(s * (STAGE / 16));
+          const uint32_t b0 = STREAM ? blo + (smem_u32(ring + s * STAGE + CH * P * 16) >> 4)
+                                     : w0 + uint32_t(kb * CH * BN);
+          auto mma = [&](int t, int kk, int m, auto accumulate) {
+            const uint32_t at = a0 + uint32_t((t / 3) * W2 + t % 3 + 2 * kk * P);  // tap's position 0
+            const uint32_t bt = b0 + (STREAM ? uint32_t((t * CH + 2 * kk) * 8)
+                                             : uint32_t((t * kch + 2 * kk) * BN));
+            umma_go<decltype(accumulate)::value>(acc + uint32_t(m * BN), desc_at(at + m * 128, AHI),
+                                                 desc_at(bt, BHI), idesc);
           };
-          if (kb == 0)
-            tap(0, std::true_type{});
-          else
-            tap(0, std::false_type{});
+          if (NBUF == 1 && kb == 0) {
+            // block by block, as the epilogue empties them
 #pragma unroll 1
-          for (int t = 1; t < 9; ++t) tap(t, std::false_type{});
+            for (int m = 0; m < MT && !bad; ++m) {
+              if (!tma::mbar_wait(&tempty[m], eph)) {
+                bad = true;
+                break;
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              mma(0, 0, m, std::false_type{});
+#pragma unroll
+              for (int t = 0; t < 9; ++t)
+#pragma unroll
+                for (int kk = 0; kk < CB / 16; ++kk)
+                  if (t > 0 || kk > 0) mma(t, kk, m, std::true_type{});
+            }
+          } else {
+            // consecutive MMAs go to different blocks
+            if (NBUF == 2 && kb == 0) {
+              for (int m = 0; m < MT; ++m) bad |= !tma::mbar_wait(&tempty[b * MT + m], eph);
+              if (bad) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+              for (int m = 0; m < MT; ++m) mma(0, 0, m, std::false_type{});
+            } else {
+#pragma unroll
+              for (int m = 0; m < MT; ++m) mma(0, 0, m, std::true_type{});
+            }
+#pragma unroll
+            for (int kk = 1; kk < CB / 16; ++kk)
+#pragma unroll
+              for (int m = 0; m < MT; ++m) mma(0, kk, m, std::true_type{});
+#pragma unroll 1
+            for (int t = 1; t < 9; ++t)
+#pragma unroll
+              for (int kk = 0; kk < CB / 16; ++kk)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) mma(t, kk, m, std::true_type{});
+          }
           umma_commit(&empty[s]);
           if (++s == S) {
             s = 0;
@@ -324,8 +365,8 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
     const bool wide = p.wide != 0;
     int it = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
-      const int b = it & 1;
-      bool ok = tma::mbar_wait(&tfull[b], uint32_t((it >> 1) & 1));
+      const int b = it % NBUF;
+      bool ok = tma::mbar_wait(&tfull[b], uint32_t((it / NBUF) & 1));
       ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is warp-collective
       if (!ok) {
         bad = true;
@@ -351,11 +392,9 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
         __syncwarp();
         tmem_ld32(tmem + (uint32_t(lq) << 16) + uint32_t(b * ACC + m * BN + c * 32), v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (k == UNITS / G - 1) {
-          // the accumulator is in registers: it may be overwritten
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          warp_arrive(&tempty[b], lane);
-        }
+        // the block's share is in registers: it may be overwritten
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        warp_arrive(&tempty[b * MT + m], lane);
         if (store) {
           const float4* const bias = reinterpret_cast<const float4*>(bsm + c * 32);
 #pragma unroll
@@ -390,35 +429,38 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == MMA_WARP)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(2 * ACC));
+                 "r"(TT::COLS));
   if (bad) atomicExch(err, 1);
 }
 
-// Shared memory of a launch with tiles of M positions and BN output channels,
-// and the stages it leaves room for (0: it does not fit).
-inline int flow_stages(int M, int BN, int cin, int wid, int* P) {
-  const int q = (M + 2 * (wid + 3) + 7) / 8 * 8;  // M positions and the taps' reach
-  *P = q;
-  const int weights = 9 * cin * BN * 2, stage = FL_CH * q * 16;
-  const int s = (FL_SMEM - weights) / stage;
-  return weights >= FL_SMEM ? 0 : s > FL_SMAX ? FL_SMAX : s;
+// Positions of a strip and stages of the ring that fit beside the weights (0:
+// fewer than two do not).
+template <int BN, int MT, bool STREAM>
+int flow_stages(int cin, int wid, int* P) {
+  using TT = FlowTile<BN, MT, STREAM>;
+  *P = (TT::M + 2 * (wid + 3) + 7) / 8 * 8;  // M positions and the taps' reach
+  const int weights = STREAM ? 0 : 9 * cin * BN * 2;
+  const int s = (FL_SMEM - weights) / (TT::CH * *P * 16 + TT::WSTAGE);
+  return weights >= FL_SMEM || s < 2 ? 0 : s > FL_SMAX ? FL_SMAX : s;
 }
 
-template <int BN, int MT>
+// SP_EINVAL where it does not fit
+template <int BN, int MT, bool STREAM = false>
 int launch_flow(FlowParams p, int* err, cudaStream_t s) {
-  using TT = FlowTile<BN, MT>;
-  p.S = flow_stages(TT::M, BN, p.cin, p.wid, &p.P);
-  if (p.S < 2) return SP_EINVAL;
-  const int smem = 9 * p.cin * BN * 2 + p.S * FL_CH * p.P * 16 + 1024;
+  using TT = FlowTile<BN, MT, STREAM>;
+  if (p.cin % TT::CB != 0) return SP_EINVAL;
+  p.S = flow_stages<BN, MT, STREAM>(p.cin, p.wid, &p.P);
+  if (p.S == 0) return SP_EINVAL;
+  const int smem = (STREAM ? 0 : 9 * p.cin * BN * 2) + p.S * (TT::CH * p.P * 16 + TT::WSTAGE) + 1024;
   const cudaError_t attr =
-      cudaFuncSetAttribute(k_conv3x3_flow<BN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           227 * 1024);
+      cudaFuncSetAttribute(k_conv3x3_flow<BN, MT, STREAM>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (attr != cudaSuccess) return SP_ECUDA;
   const long long QN = (long long)(p.h + 2) * (p.wid + 2) * p.n;
   p.tiles = int((QN + TT::M - 1) / TT::M);
   const int ny = p.cout / BN, gx = sms() / ny > 0 ? sms() / ny : 1;
-  k_conv3x3_flow<BN, MT><<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)), FL_NT, smem,
-                           s>>>(p, err);
+  k_conv3x3_flow<BN, MT, STREAM><<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)),
+                                   FL_NT, smem, s>>>(p, err);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 

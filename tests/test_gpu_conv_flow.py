@@ -1,6 +1,6 @@
-"""The persistent tcgen05 convolution (weights resident in shared memory): each
-of its tiles (32, 64 and 128 outputs; 1024, 512 and 256 positions), K loops of
-one to eight stages, images smaller than a tile and than a strip's reach,
+"""The persistent tcgen05 convolution (weights resident in shared memory, or
+streamed): each of its tiles (32, 64 and 128 outputs; 1024, 512 and 256
+positions), K loops of one to sixteen stages, images smaller than a tile and than a strip's reach,
 several tiles a CTA, outputs that start on 16 but not on 32 bytes, every set of
 epilogue operands -- against a float64 reference on the same bf16 operands.
 The sums are exact to K 2^-24 of their magnitude, the stored pre-activation to
@@ -32,7 +32,10 @@ def conv64(x, w):
 @pytest.mark.parametrize("n,h,w,ci,co", [
     (1, 1, 1, 32, 32), (1, 2, 3, 32, 64), (3, 33, 17, 64, 32), (2, 70, 300, 32, 32),
     (1, 40, 400, 128, 32), (5, 67, 67, 64, 64), (2, 20, 130, 128, 64), (2, 31, 64, 64, 128),
-    (1, 9, 11, 32, 256), (40, 100, 101, 32, 32), (1, 16, 16, 256, 32), (2, 128, 128, 32, 64)])
+    (1, 9, 11, 32, 256), (40, 100, 101, 32, 32), (1, 16, 16, 256, 32), (2, 128, 128, 32, 64),
+    # weights streamed: one and several tiles a CTA, K blocks of 16 channels, two
+    # output blocks, a strip wider than its tile
+    (1, 5, 7, 128, 128), (2, 130, 130, 144, 128), (1, 33, 17, 256, 256), (1, 6, 640, 128, 128)])
 @pytest.mark.parametrize("ops", ["bias,res,z,a", "a", "z"])
 def test_flow_convolution(n, h, w, ci, co, ops):
     torch.manual_seed(h * w + ci)
