@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(OUT1_NT, 2)
     k_conv3x3_out1(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ bias, float* __restrict__ out, int h, int wid) {
   constexpr int GL = CIN / 8, COLS = OUT1_NT / GL;  // lanes a pixel, columns of a CTA
-  __shared__ float vs[2][3][COLS];
+  constexpr int RB = 4;  // rows between barriers
+  __shared__ float vs[2][RB][3][COLS];
   const int c0 = (threadIdx.x % GL) * 8, col = threadIdx.x / GL;
   const int x0 = blockIdx.x * (COLS - 2), y0 = blockIdx.y * OUT1_R;
   const long long img = blockIdx.z;
@@ -132,12 +133,9 @@ __global__ void __launch_bounds__(OUT1_NT, 2)
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int d = 0; d < 3; ++d) s[i][d] = make_float2(0.f, 0.f);
-  uint4 n1 = load(y0 - 1), n2 = load(y0), n3 = load(y0 + 1);  // rows in flight
-  for (int y = y0 - 1; y <= ye; ++y) {
-    const uint4 cur = n1;
-    n1 = n2;
-    n2 = n3;
-    n3 = load(y + 3);
+  // one row of x: it adds to three output rows; `t`, if not null, gets the column
+  // sums of output row y - 1, which is then complete
+  auto row = [&](const uint4& cur, float* t) {
     const float2 v[4] = {f2bf(cur.x), f2bf(cur.y), f2bf(cur.z), f2bf(cur.w)};
     // row y is the lower row (dy = +1) of output y - 1, the centre of y, the
     // upper row (dy = -1) of y + 1
@@ -147,27 +145,44 @@ __global__ void __launch_bounds__(OUT1_NT, 2)
       for (int d = 0; d < 3; ++d)
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[i][d] = __ffma2_rn(wt[(2 - i) * 3 + d][e], v[e], s[i][d]);
-    const int o = y - 1, buf = y & 1;
-    if (o >= y0) {
+    if (t) {
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        float t = s[0][d].x + s[0][d].y;
+        float u = s[0][d].x + s[0][d].y;
 #pragma unroll
-        for (int m = GL / 2; m > 0; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
-        if (threadIdx.x % GL == 0) vs[buf][d][col] = t;
+        for (int m = GL / 2; m > 0; m >>= 1) u += __shfl_xor_sync(0xffffffffu, u, m);
+        if (threadIdx.x % GL == 0) t[d * COLS + col] = u;
       }
-    }
-    __syncthreads();
-    if (o >= y0 && threadIdx.x < COLS - 2 && x0 + int(threadIdx.x) < wid) {
-      const int q = threadIdx.x + 1;  // column of output x0 + threadIdx.x
-      out[(img * h + o) * wid + x0 + threadIdx.x] =
-          b + ((vs[buf][0][q - 1] + vs[buf][1][q]) + vs[buf][2][q + 1]);
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       s[0][d] = s[1][d];
       s[1][d] = s[2][d];
       s[2][d] = make_float2(0.f, 0.f);
+    }
+  };
+  row(load(y0 - 1), nullptr);
+  row(load(y0), nullptr);
+  uint4 nx[RB];  // the next rows, in flight
+#pragma unroll
+  for (int k = 0; k < RB; ++k) nx[k] = load(y0 + 1 + k);
+  int buf = 0;
+  for (int o = y0; o < ye; o += RB, buf ^= 1) {
+    uint4 cur[RB];
+#pragma unroll
+    for (int k = 0; k < RB; ++k) cur[k] = nx[k];
+#pragma unroll
+    for (int k = 0; k < RB; ++k) nx[k] = load(o + RB + 1 + k);
+#pragma unroll
+    for (int k = 0; k < RB; ++k) row(cur[k], &vs[buf][k][0][0]);
+    // one barrier: the other buffer's readers passed the one before
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < (RB * COLS + OUT1_NT - 1) / OUT1_NT; ++k) {
+      const int i = threadIdx.x + k * OUT1_NT, r = i / COLS, c = i - r * COLS;
+      if (r < RB && c < COLS - 2 && x0 + c < wid && o + r < ye)
+        out[(img * h + o + r) * wid + x0 + c] =
+            b + ((vs[buf][r][0][c] + vs[buf][r][1][c + 1]) + vs[buf][r][2][c + 2]);
     }
   }
 }
