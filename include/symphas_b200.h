@@ -197,9 +197,10 @@ int sp_reduce(sp_handle* h, int inst, int field, double* mass, double* energy);
  * process start with it.  No counterpart in SymPhas. */
 int sp_autotune(sp_handle* h, int reps);
 /* Steps one launch of the chosen kernel advances (its temporal-block depth):
- * 1 for the one-step kernels; k > 1 for a temporally blocked 2D kernel, which
- * sp_step then launches once per k steps (and once with fewer steps for a
- * remainder).  No counterpart in SymPhas (SolverFT takes one step per call of
+ * 1 for the one-step kernels; k > 1 for a temporally blocked 2D kernel, or on a
+ * 2D grid that one wave of CTAs covers, where sp_step launches once per k steps
+ * (and once with fewer steps for a remainder; a single step takes the one-step
+ * shape that sp_kernel_info describes).  No counterpart in SymPhas (SolverFT takes one step per call of
  * Solver::step, examples/solvers/solverft.h:46-103). */
 int sp_steps_per_launch(const sp_handle* h, int* kt);
 /* The chosen kernel shape: {tile x, tile y, rows per thread, TMA stages in
@@ -272,7 +273,9 @@ int sp_conv_tc_status(int* gave_up);
  * memory (the CTA shape is chosen per layer class; SP_STRIP_SHAPE="mt,cb,s"
  * fixes it for timing),
  * the weights re-tiled into `wt` (9 cin cout bf16 of scratch, device memory)
- * and loaded with one bulk copy per channel block.  cin a multiple of 16,
+ * and loaded with one bulk copy per channel block.  Where the weights and two
+ * strips fit in shared memory (cin a multiple of 32) a persistent kernel with
+ * resident weights runs instead and leaves `wt` alone.  cin a multiple of 16,
  * cout 32, 64 or a multiple of 128, w_ <= 764, bias 16-byte aligned; bounded
  * waits report through sp_conv_tc_status. */
 int sp_conv3x3_fwd_strip(const void* x, const void* w, void* wt, const float* bias,
