@@ -317,7 +317,7 @@ int sp_conv3x3_out1(const void* x, const void* w, const float* bias, float* out,
 /* The element-wise backward of a layer: dz [npix][c] (bf16) = da * gelu'(z)
  * (tanh form) and db [c] (fp32, or null) += the sums of dz over the pixels;
  * with z null dz is not written and db gets the sums of da.  c a multiple of
- * 8, at most 2048; z, da, dz 16-byte aligned.  No counterpart in SymPhas. */
+ * 8; z, da, dz 16-byte aligned.  No counterpart in SymPhas. */
 int sp_gelu_bwd_bf16(const void* z, const void* da, void* dz, float* db, long long npix, int c,
                      void* stream);
 /* wf [cin][3][3][cout] = w [cout][3][3][cin] rotated by 180 degrees: the input

@@ -206,8 +206,9 @@ constexpr int GB_NT = 256;
 template <bool Z>
 __global__ void __launch_bounds__(GB_NT)
     k_gelu_bwd(const __nv_bfloat16* __restrict__ z, const __nv_bfloat16* __restrict__ da,
-               __nv_bfloat16* __restrict__ dz, float* __restrict__ db, long long npix, int c) {
+               __nv_bfloat16* __restrict__ dz, float* __restrict__ db, long long npix, int cs) {
   extern __shared__ float sums[];  // [rows of a block][c]
+  const int c0 = blockIdx.y * 8 * GB_NT, c = min(cs - c0, 8 * GB_NT);  // this CTA's channels
   const int cg = c / 8, rows = GB_NT / cg;
   const int g = threadIdx.x % cg, r = threadIdx.x / cg;
   float acc[8];
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(GB_NT)
 #pragma unroll
       for (int k = 0; k < U; ++k)
         if (p + k * step < npix) {
-          const long long o = (p + k * step) * c + g * 8;
+          const long long o = (p + k * step) * cs + c0 + g * 8;
           d[k] = __ldg(reinterpret_cast<const uint4*>(da + o));
           if constexpr (Z) zz[k] = __ldg(reinterpret_cast<const uint4*>(z + o));
         }
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(GB_NT)
             const float2 f = f2bf(zv[e]), y = f2bf(dv[e]);
             dv[e] = bf2(y.x * gelu_grad(f.x), y.y * gelu_grad(f.y));
           }
-          *reinterpret_cast<uint4*>(dz + (p + k * step) * c + g * 8) = d[k];
+          *reinterpret_cast<uint4*>(dz + (p + k * step) * cs + c0 + g * 8) = d[k];
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(GB_NT)
   for (int i = threadIdx.x; i < c; i += GB_NT) {
     float t = 0.f;
     for (int k = 0; k < rows; ++k) t += sums[k * c + i];
-    atomicAdd(db + i, t);
+    atomicAdd(db + c0 + i, t);
   }
 }
 
@@ -297,15 +298,19 @@ extern "C" int sp_conv3x3_out1(const void* x, const void* w, const float* bias, 
 extern "C" int sp_gelu_bwd_bf16(const void* z, const void* da, void* dz, float* db, long long npix,
                                 int c, void* stream) {
   using namespace sp::conv;
-  if (!da || npix < 1 || c < 8 || c % 8 != 0 || c > 8 * GB_NT || !al16(da) || !al16(z) ||
+  if (!da || npix < 1 || c < 8 || c % 8 != 0 || !al16(da) || !al16(z) ||
       !al16(dz) || (z ? !dz : !db))
     return SP_EINVAL;
-  const int rows = GB_NT / (c / 8);
+  // blocks of at most 2048 channels (one lane group of 8 a thread)
+  const int cb = c < 8 * GB_NT ? c : 8 * GB_NT, ny = (c + 8 * GB_NT - 1) / (8 * GB_NT);
+  if (ny > 65535) return SP_EINVAL;
+  const int rows = GB_NT / (cb / 8);
   const long long want = (npix + rows - 1) / rows;
   const long long most = 6LL * sms();  // 6 CTAs an SM: each adds its c sums once
   auto kern = z ? k_gelu_bwd<true> : k_gelu_bwd<false>;
-  kern<<<unsigned(want < most ? want : most), GB_NT, rows * c * int(sizeof(float)),
-               static_cast<cudaStream_t>(stream)>>>(
+  // a row of sums per pixel lane: 8 KB at most, whatever the channel count
+  kern<<<dim3(unsigned(want < most ? want : most), unsigned(ny)), GB_NT,
+         8 * GB_NT * int(sizeof(float)), static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(z), static_cast<const __nv_bfloat16*>(da),
       static_cast<__nv_bfloat16*>(dz), db, npix, c);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;

@@ -70,7 +70,7 @@ def test_last_layer(n, h, w, ci):
                                    stream()) == C.SP_EINVAL
 
 
-@pytest.mark.parametrize("npix,c", [(1, 8), (7, 24), (1000, 32), (33, 256), (5, 2048), (70000, 64)])
+@pytest.mark.parametrize("npix,c", [(1, 8), (7, 24), (1000, 32), (33, 256), (5, 2048), (9, 2056), (70000, 64)])
 def test_gelu_backward_and_bias_gradient(npix, c):
     torch.manual_seed(c)
     z = (3 * torch.randn(npix, c, device="cuda")).bfloat16()
