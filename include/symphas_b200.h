@@ -276,8 +276,9 @@ int sp_conv_tc_status(int* gave_up);
  * and loaded with one bulk copy per channel block.  Where the weights and two
  * strips fit in shared memory (cin a multiple of 32) a persistent kernel with
  * resident weights runs instead and leaves `wt` alone.  cin a multiple of 16,
- * cout 32, 64 or a multiple of 128, w_ <= 764, bias 16-byte aligned; bounded
- * waits report through sp_conv_tc_status. */
+ * cout 32, 64 or a multiple of 128, w_ <= 764; x, wt, bias, z and a 16-byte
+ * aligned, res on 4 bytes, w any (w or res off 16 bytes keep the strip
+ * kernel); bounded waits report through sp_conv_tc_status. */
 int sp_conv3x3_fwd_strip(const void* x, const void* w, void* wt, const float* bias,
                          const void* res, void* z, void* a, int n, int h, int w_, int cin,
                          int cout, void* stream);

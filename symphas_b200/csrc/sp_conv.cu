@@ -1138,12 +1138,14 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
   int* err = tc_error_flag();
   if (!err) return SP_ENOMEM;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!getenv("SP_STRIP_SHAPE")) {
-    const auto al = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 32 == 0; };
+  // the persistent kernel copies w and reads res 16 bytes at a time; the strip
+  // kernel re-tiles w one element at a time and reads res by pairs of channels
+  const auto on = [](const void* q, int b) { return reinterpret_cast<uintptr_t>(q) % b == 0; };
+  if (!getenv("SP_STRIP_SHAPE") && on(w, 16) && on(res, 16)) {
     FlowParams f{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), bias,
                  static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(z),
                  static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout, 0, 0, 0, up,
-                 al(res) && al(z) && al(a)};
+                 on(res, 32) && on(z, 32) && on(a, 32)};
     const int rc = flow_fwd(f, wt, err, s);
     if (rc != SP_EINVAL) return rc;
   }

@@ -6,6 +6,7 @@ epilogue operands -- against a float64 reference on the same bf16 operands.
 The sums are exact to K 2^-24 of their magnitude, the stored pre-activation to
 one bf16 rounding (2^-8) more, the activation to tanh.approx's 2^-11 more."""
 import ctypes
+import math
 
 import pytest
 import torch
@@ -62,3 +63,32 @@ def test_flow_convolution(n, h, w, ci, co, ops):
     for got, want in ((z, zr), (a, F.gelu(zr, approximate="tanh"))):
         if got is not None:
             assert torch.allclose(got.double(), want, rtol=2.0 ** -7, atol=2e-3)
+
+
+@pytest.mark.parametrize("ci,co", [(32, 32), (32, 64), (128, 128)])
+@pytest.mark.parametrize("off_w,off_res", [(1, 0), (0, 2), (8, 2), (3, 6)])
+@pytest.mark.parametrize("up", [False, True])
+def test_weights_and_residual_off_16_bytes(ci, co, off_w, off_res, up):
+    """w on any element and res on any pair of channels (offsets in elements of
+    bf16): such calls keep the strip kernel, whose accesses are that narrow."""
+    torch.manual_seed(ci + co)
+    n, h, w = 2, 12, 18
+    x = torch.randn(n, h // 2 if up else h, w // 2 if up else w, ci, device="cuda").bfloat16()
+    xr = x.repeat_interleave(2, 1).repeat_interleave(2, 2) if up else x
+
+    def at(shape, off, scale):
+        buf = (scale * torch.randn(math.prod(shape) + off, device="cuda")).bfloat16()
+        return buf[off:].view(shape)
+
+    wt = at((co, 3, 3, ci), off_w, 1 / (3 * ci ** 0.5))
+    res = at((n, h, w, co), off_res, 1.0)
+    assert (wt.data_ptr() % 16 or res.data_ptr() % 16) and res.data_ptr() % 4 == 0
+    scratch = torch.empty(9 * ci * co, device="cuda", dtype=torch.bfloat16)
+    z = torch.full((n, h, w, co), float("nan"), device="cuda", dtype=torch.bfloat16)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    fwd = C.lib().sp_conv3x3_fwd_strip_up2 if up else C.lib().sp_conv3x3_fwd_strip
+    assert fwd(ptr(x), ptr(wt), ptr(scratch), None, ptr(res), ptr(z), None, n, h, w, ci, co,
+               s) == C.SP_OK
+    flag = ctypes.c_int(-1)
+    assert C.lib().sp_conv_tc_status(ctypes.byref(flag)) == C.SP_OK and flag.value == 0
+    assert torch.allclose(z.double(), conv64(xr, wt) + res.double(), rtol=2.0 ** -7, atol=2e-3)
