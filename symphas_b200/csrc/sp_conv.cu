@@ -932,7 +932,8 @@ __global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p, in
         }
       }
     }
-    for (int ks = 0; ks < nk && !bad; ++ks) {
+    int fills = 0;
+    for (int ks = 0; ks < nk && !bad; ++ks, ++fills) {
       const int s = ks % S;
       if (ks >= S && !tma::mbar_wait(&empty[s], uint32_t((ks / S - 1) & 1))) {
         bad = true;
@@ -960,6 +961,8 @@ __global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p, in
                    : "memory");
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    // (bulk copies that the MMA warp, having given up, did not wait for)
+    if (tid == 0) tma::drain(full, S, fills > S ? fills - S : 0, fills - 1);
 
     // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 of the
     // M-tiles m = w / 4, w / 4 + 2

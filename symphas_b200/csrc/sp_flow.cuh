@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
     constexpr int LP = 32 / CH, STEP = FL_PROD / CH;
     const int j = lane / LP, lp = warp * LP + lane % LP;
     const int sy = STEP / W2, sx = STEP - sy * W2;
-    int s = 0;
+    int s = 0, fills = 0;
     uint32_t ph = 1;  // a fresh barrier passes the wait for the phase before its first
     for (int tile = blockIdx.x; tile < p.tiles && !bad; tile += gridDim.x) {
       // strip position 0 is output position tile * M - (W2 + 1); counted from
@@ -266,12 +266,16 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
         asm volatile("cp.async.wait_all;" ::: "memory");
         tma::fence_proxy_async();
         warp_arrive(&full[s], lane);
+        ++fills;
         if (++s == S) {
           s = 0;
           ph ^= 1;
         }
       }
     }
+    // the MMA warp waits for every fill it uses; where it gave up, the bulk
+    // copies of the last S fills may still be in flight
+    if (STREAM && tid == 0) tma::drain(full, S, fills > S ? fills - S : 0, fills - 1);
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
       // ---- MMA issuer: per stage, for every tap and K step of 16 channels,
