@@ -516,6 +516,10 @@ namespace conv {
 
 constexpr int TC_BM = 128, TC_BK = 64;
 
+// set by a tcgen05 CTA that gave up on a wait (one for each GPU; nothing is
+// allocated, so a first call may be part of a stream capture)
+__device__ int tc_gave_up;
+
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
   // K-major, no swizzle: start >> 4, LBO = 128 B, SBO = 1024 B, version 1
   return uint64_t((saddr >> 4) & 0x3FFF) | (uint64_t(128 >> 4) << 16) |
@@ -574,7 +578,7 @@ struct TcTile {
 // the MMAs of each stage once full[s] completes, committing to empty[s] (the
 // stage may be refilled) and, after the last, to done.
 template <int BN>
-__global__ void __launch_bounds__(160) k_conv3x3_fwd_tc(const FwdParams p, int* err) {
+__global__ void __launch_bounds__(160) k_conv3x3_fwd_tc(const FwdParams p) {
   using TT = TcTile<BN>;
   constexpr int S = TT::S;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -718,42 +722,32 @@ __global__ void __launch_bounds__(160) k_conv3x3_fwd_tc(const FwdParams p, int* 
   if (warp == 4)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(TT::COLS));
-  if (bad) atomicExch(err, 1);
-}
-
-// device flag set by a tcgen05 CTA that gave up on a wait (allocated once)
-int* tc_error_flag() {
-  static int* e = [] {
-    int* f = nullptr;
-    if (cudaMalloc(&f, sizeof(int)) != cudaSuccess) return static_cast<int*>(nullptr);
-    cudaMemset(f, 0, sizeof(int));
-    return f;
-  }();
-  return e;
+  if (bad) atomicExch(&tc_gave_up, 1);
 }
 
 }  // namespace conv
 }  // namespace sp
 
 extern "C" int sp_conv_tc_status(int* gave_up) {
-  int* err = sp::conv::tc_error_flag();
-  if (!err || !gave_up) return SP_EINVAL;
+  const int zero = 0;
+  if (!gave_up) return SP_EINVAL;
   if (cudaDeviceSynchronize() != cudaSuccess) return SP_ECUDA;
-  if (cudaMemcpy(gave_up, err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+  if (cudaMemcpyFromSymbol(gave_up, sp::conv::tc_gave_up, sizeof(int)) != cudaSuccess)
     return SP_ECUDA;
-  return cudaMemset(err, 0, sizeof(int)) == cudaSuccess ? SP_OK : SP_ECUDA;
+  return cudaMemcpyToSymbol(sp::conv::tc_gave_up, &zero, sizeof(int)) == cudaSuccess ? SP_OK
+                                                                                    : SP_ECUDA;
 }
 
 namespace sp {
 namespace conv {
 template <int BN>
-int launch_fwd_tc(const FwdParams& p, int* err, cudaStream_t s) {
+int launch_fwd_tc(const FwdParams& p, cudaStream_t s) {
   static const cudaError_t attr = cudaFuncSetAttribute(
       k_conv3x3_fwd_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcTile<BN>::SMEM);
   if (attr != cudaSuccess) return SP_ECUDA;
   const long long npix = (long long)p.n * p.h * p.wid;
   k_conv3x3_fwd_tc<BN><<<dim3(unsigned((npix + TC_BM - 1) / TC_BM), unsigned(p.cout / BN)), 160,
-                         TcTile<BN>::SMEM, s>>>(p, err);
+                         TcTile<BN>::SMEM, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 }  // namespace conv
@@ -766,15 +760,13 @@ extern "C" int sp_conv3x3_fwd_tc(const void* x, const void* w, const float* bias
   if (!x || !w || (!z && !a) || n < 1 || h < 1 || w_ < 1 || cin % 8 != 0 || cin < 8 ||
       !(cout == 32 || cout % 64 == 0))
     return SP_EINVAL;
-  int* err = tc_error_flag();
-  if (!err) return SP_ENOMEM;
   FwdParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), bias,
               static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(z),
               static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout};
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cout == 32) return launch_fwd_tc<32>(p, err, s);
-  if (cout % 128 == 0) return launch_fwd_tc<128>(p, err, s);
-  return launch_fwd_tc<64>(p, err, s);
+  if (cout == 32) return launch_fwd_tc<32>(p, s);
+  if (cout % 128 == 0) return launch_fwd_tc<128>(p, s);
+  return launch_fwd_tc<64>(p, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -867,7 +859,7 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 template <int BN, int CB, int MT>
-__global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p, int* err) {
+__global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p) {
   using TT = StripTile<BN, CB, MT>;
   constexpr int ST_MT = MT, ST_M = TT::M;
   constexpr int CH = TT::CH;
@@ -1057,11 +1049,11 @@ __global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p, in
   if (warp == 8)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(TT::COLS));
-  if (bad) atomicExch(err, 1);
+  if (bad) atomicExch(&tc_gave_up, 1);
 }
 
 template <int BN, int CB, int MT>
-int launch_strip(StripParams p, int* err, cudaStream_t s, int smax) {
+int launch_strip(StripParams p, cudaStream_t s, int smax) {
   using TT = StripTile<BN, CB, MT>;
   constexpr int ST_M = TT::M;
   const int W2 = p.wid + 2;
@@ -1087,7 +1079,7 @@ int launch_strip(StripParams p, int* err, cudaStream_t s, int smax) {
   if (attr != cudaSuccess) return SP_ECUDA;
   const long long QN = (long long)(p.h + 2) * W2 * p.n;
   k_conv3x3_strip<BN, CB, MT><<<dim3(unsigned((QN + ST_M - 1) / ST_M), unsigned(p.cout / BN)),
-                                ST_NT, smem, s>>>(p, err);
+                                ST_NT, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 
@@ -1101,24 +1093,24 @@ namespace {
 // largest tile that leaves room for two strips (a strip's reach beyond its tile,
 // two rows, is gathered again by the next tile), with the weights resident, or
 // streamed from `wt` where they do not fit
-int flow_fwd(sp::conv::FlowParams p, void* wt, int* err, cudaStream_t s) {
+int flow_fwd(sp::conv::FlowParams p, void* wt, cudaStream_t s) {
   using namespace sp::conv;
   int rc = SP_EINVAL;
   if (p.cout == 32) {
-    rc = launch_flow<32, 8>(p, err, s);
-    if (rc == SP_EINVAL) rc = launch_flow<32, 4>(p, err, s);
+    rc = launch_flow<32, 8>(p, s);
+    if (rc == SP_EINVAL) rc = launch_flow<32, 4>(p, s);
   } else if (p.cout == 64) {
-    rc = launch_flow<64, 4>(p, err, s);
-    if (rc == SP_EINVAL) rc = launch_flow<64, 2>(p, err, s);
+    rc = launch_flow<64, 4>(p, s);
+    if (rc == SP_EINVAL) rc = launch_flow<64, 2>(p, s);
   } else if (p.cout % 128 == 0) {
-    rc = launch_flow<128, 2>(p, err, s);
+    rc = launch_flow<128, 2>(p, s);
     int P;
     if (rc == SP_EINVAL && p.cin % FL_CBS == 0 && flow_stages<128, 4, true>(p.cin, p.wid, &P)) {
       k_tile_weights<<<256, 256, 0, s>>>(p.w, static_cast<__nv_bfloat16*>(wt), p.cin, p.cout, 128,
                                           FL_CBS);
       if (cudaGetLastError() != cudaSuccess) return SP_ECUDA;
       p.w = static_cast<const __nv_bfloat16*>(wt);
-      rc = launch_flow<128, 4, true>(p, err, s);
+      rc = launch_flow<128, 4, true>(p, s);
     }
   }
   return rc;
@@ -1138,8 +1130,6 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
   // every padded position (with a strip's reach past the end) below 2^31
   if ((long long)n * h * w_ * cin >= (1LL << 31)) return SP_EINVAL;
   if ((long long)n * (h + 2) * (w_ + 2) + 4LL * (w_ + 3) + 4096 >= (1LL << 31)) return SP_EINVAL;
-  int* err = tc_error_flag();
-  if (!err) return SP_ENOMEM;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   // the persistent kernel copies w and reads res 16 bytes at a time; the strip
   // kernel re-tiles w one element at a time and reads res by pairs of channels
@@ -1149,7 +1139,7 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
                  static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(z),
                  static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout, 0, 0, 0, up,
                  on(res, 32) && on(z, 32) && on(a, 32)};
-    const int rc = flow_fwd(f, wt, err, s);
+    const int rc = flow_fwd(f, wt, s);
     if (rc != SP_EINVAL) return rc;
   }
   const int bn = cout == 32 ? 32 : cout == 64 ? 64 : 128;
@@ -1189,8 +1179,8 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
                 static_cast<__nv_bfloat16*>(a), n, h, w_, cin, cout, 0, 0, up};
   auto go = [&](auto bn_c, auto cb_c) {
     constexpr int BN = decltype(bn_c)::value, CB = decltype(cb_c)::value;
-    return mt == 2 ? launch_strip<BN, CB, 2>(p, err, s, smax)
-                   : launch_strip<BN, CB, 4>(p, err, s, smax);
+    return mt == 2 ? launch_strip<BN, CB, 2>(p, s, smax)
+                   : launch_strip<BN, CB, 4>(p, s, smax);
   };
   using I32 = std::integral_constant<int, 32>;
   using I16 = std::integral_constant<int, 16>;
@@ -1225,12 +1215,10 @@ extern "C" int sp_conv3x3_wgrad(const void* x, const void* dy, float* dw, int n,
   const long long npix = (long long)n * h * w_;
   if (npix >= (1LL << 31)) return SP_EINVAL;  // the kernel's pixel arithmetic is 32-bit
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int* err = tc_error_flag()) {
-    WgParams t{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw,
-               n, h, w_, cin, cout, 0, 0, 0, 0, 0, reinterpret_cast<uintptr_t>(dw) % 16 == 0};
-    const int rc = wgrad_tc(t, err, s);
-    if (rc != SP_EINVAL) return rc;
-  }
+  WgParams t{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw,
+             n, h, w_, cin, cout, 0, 0, 0, 0, 0, reinterpret_cast<uintptr_t>(dw) % 16 == 0};
+  const int rc = wgrad_tc(t, s);
+  if (rc != SP_EINVAL) return rc;
   const unsigned gx = unsigned(9 * (cin / WM)), gy = unsigned((cout + WN - 1) / WN);
   // enough pixel chunks for about four waves of CTAs
   long long want = (long long)sms() * 8 / (gx * gy);

@@ -168,7 +168,7 @@ struct FlowTile {
 };
 
 template <int BN, int MT, bool STREAM>
-__global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, int* err) {
+__global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p) {
   using TT = FlowTile<BN, MT, STREAM>;
   constexpr int M = TT::M, ACC = TT::ACC, NBUF = TT::NBUF, CB = TT::CB, CH = TT::CH;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p, i
   if (warp == MMA_WARP)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(TT::COLS));
-  if (bad) atomicExch(err, 1);
+  if (bad) atomicExch(&tc_gave_up, 1);
 }
 
 // Positions of a strip and stages of the ring that fit beside the weights (0:
@@ -450,7 +450,7 @@ int flow_stages(int cin, int wid, int* P) {
 
 // SP_EINVAL where it does not fit
 template <int BN, int MT, bool STREAM = false>
-int launch_flow(FlowParams p, int* err, cudaStream_t s) {
+int launch_flow(FlowParams p, cudaStream_t s) {
   using TT = FlowTile<BN, MT, STREAM>;
   if (p.cin % TT::CB != 0) return SP_EINVAL;
   p.S = flow_stages<BN, MT, STREAM>(p.cin, p.wid, &p.P);
@@ -464,7 +464,7 @@ int launch_flow(FlowParams p, int* err, cudaStream_t s) {
   p.tiles = int((QN + TT::M - 1) / TT::M);
   const int ny = p.cout / BN, gx = sms() / ny > 0 ? sms() / ny : 1;
   k_conv3x3_flow<BN, MT, STREAM><<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)),
-                                   FL_NT, smem, s>>>(p, err);
+                                   FL_NT, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 

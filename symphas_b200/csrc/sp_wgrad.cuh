@@ -59,7 +59,7 @@ struct WgTile {
 };
 
 template <int COB, int N>
-__global__ void __launch_bounds__(WG_NT, 1) k_wgrad_tc(const WgParams p, int* err) {
+__global__ void __launch_bounds__(WG_NT, 1) k_wgrad_tc(const WgParams p) {
   using TT = WgTile<COB, N>;
   constexpr int CHO = TT::CHO, CHX = TT::CHX, HALO = TT::HALO, NV = TT::NV, VR = TT::VR;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -243,11 +243,11 @@ __global__ void __launch_bounds__(WG_NT, 1) k_wgrad_tc(const WgParams p, int* er
   if (warp == MMA_WARP)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(TT::TCOLS));
-  if (bad) atomicExch(err, 1);
+  if (bad) atomicExch(&tc_gave_up, 1);
 }
 
 template <int COB, int N>
-int launch_wgrad(WgParams p, int* err, cudaStream_t s) {
+int launch_wgrad(WgParams p, cudaStream_t s) {
   using TT = WgTile<COB, N>;
   // columns: blocks of at most 128, of equal width up to the 16 pixels of an
   // MMA's K; rows: as many as two stages hold, at most 8 (more rows read the
@@ -278,23 +278,23 @@ int launch_wgrad(WgParams p, int* err, cudaStream_t s) {
   const int ny = TT::VSPLIT * (p.cin / N) * (p.cout / COB);
   const int gx = sms() / ny > 0 ? sms() / ny : 1;
   k_wgrad_tc<COB, N><<<dim3(unsigned(p.items < gx ? p.items : gx), unsigned(ny)), WG_NT, smem, s>>>(
-      p, err);
+      p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 
 // the tensor-memory kernel where its tiles fit the channels, else SP_EINVAL
-inline int wgrad_tc(const WgParams& p, int* err, cudaStream_t s) {
+inline int wgrad_tc(const WgParams& p, cudaStream_t s) {
   const int n = p.cin % 128 == 0 ? 128 : p.cin % 64 == 0 ? 64 : 32;
   if (p.cout == 32)
-    return n == 128 ? launch_wgrad<32, 128>(p, err, s)
-           : n == 64 ? launch_wgrad<32, 64>(p, err, s)
-                     : launch_wgrad<32, 32>(p, err, s);
+    return n == 128 ? launch_wgrad<32, 128>(p, s)
+           : n == 64 ? launch_wgrad<32, 64>(p, s)
+                     : launch_wgrad<32, 32>(p, s);
   if (p.cout == 64)
-    return n >= 64 ? launch_wgrad<64, 64>(p, err, s) : launch_wgrad<64, 32>(p, err, s);
+    return n >= 64 ? launch_wgrad<64, 64>(p, s) : launch_wgrad<64, 32>(p, s);
   if (p.cout % 128 == 0)
-    return n == 128 ? launch_wgrad<128, 128>(p, err, s)
-           : n == 64 ? launch_wgrad<128, 64>(p, err, s)
-                     : launch_wgrad<128, 32>(p, err, s);
+    return n == 128 ? launch_wgrad<128, 128>(p, s)
+           : n == 64 ? launch_wgrad<128, 64>(p, s)
+                     : launch_wgrad<128, 32>(p, s);
   return SP_EINVAL;
 }
 

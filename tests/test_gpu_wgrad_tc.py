@@ -9,6 +9,9 @@ by at most about K 2^-24 of the sum of magnitudes and by sqrt(K) 2^-24 of it
 in the mean: 1e-4 of the largest gradient is well above that for the sizes
 here (K <= 17000) and far below one wrong or missing pixel."""
 import ctypes
+import pathlib
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -67,3 +70,35 @@ def test_weight_gradient_unaligned_output():
     want = reference(x, dy, co, ci)
     got = buf[1:].view(co, 3, 3, ci).double()
     assert float((got - want).abs().max() / want.abs().max()) < 1e-4
+
+
+CAPTURED_FIRST_CALL = """
+import ctypes, torch
+from symphas_b200 import _capi as C
+p = lambda t: ctypes.c_void_p(t.data_ptr())
+torch.manual_seed(0)
+x = torch.randn(1, 12, 20, 32, device="cuda").bfloat16()
+dy = torch.randn(1, 12, 20, 64, device="cuda").bfloat16()
+dw = torch.zeros(64, 3, 3, 32, device="cuda")
+C.lib()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert C.lib().sp_conv3x3_wgrad(p(x), p(dy), p(dw), 1, 12, 20, 32, 64, s) == C.SP_OK
+g.replay()
+torch.cuda.synchronize()
+d = dy.double().reshape(-1, 64)
+for t in range(9):
+    xs = torch.roll(x.double(), (1 - t // 3, 1 - t % 3), (1, 2)).reshape(-1, 32)
+    want = d.t() @ xs
+    err = (dw[:, t // 3, t % 3].double() - want).abs().max() / want.abs().max()
+    assert float(err) < 1e-4, (t, float(err))
+"""
+
+
+def test_first_call_of_a_process_under_capture():
+    """Nothing is allocated on the way: a process whose first convolution call
+    is a weight gradient in a stream capture replays it."""
+    r = subprocess.run([sys.executable, "-c", CAPTURED_FIRST_CALL], capture_output=True, text=True,
+                       timeout=300, cwd=str(pathlib.Path(__file__).resolve().parent.parent))
+    assert r.returncode == 0, r.stderr[-2000:]
