@@ -255,8 +255,9 @@ int sp_structure_factor(sp_handle* h, int inst, int field, int threshold, double
  * activations NHWC bfloat16, work is queued on `stream` (a cudaStream_t). */
 /* z / a [n][h][w][cout] = conv3x3(x [n][h][w][cin], w [cout][3][3][cin]) with
  * circular padding, + bias (fp32, or null) + res (bf16 NHWC, or null); a gets
- * gelu(z) (tanh form); either output may be null.  cin a multiple of 32, cout
- * even. */
+ * gelu(z) (tanh form); either output may be null.  With both outputs (training)
+ * the activation is good to fp32, with a alone (inference) to tanh.approx's
+ * 2^-11.  cin a multiple of 32, cout even. */
 int sp_conv3x3_fwd(const void* x, const void* w, const float* bias, const void* res, void* z,
                    void* a, int n, int h, int w_, int cin, int cout, void* stream);
 /* The same convolution on the 5th-generation tensor cores (tcgen05.mma, fp32

@@ -75,6 +75,16 @@ __device__ __forceinline__ float gelu(float z) {
   return fmaf(hz, tanh_fast(u), hz);
 }
 
+// The same for activations that are trained through (stored beside their
+// pre-activation): 0.5 (1 + tanh u) = 1 / (1 + exp(-2 u)), which does not
+// cancel at negative z, to a few units in the last place of fp32.  Stored in
+// bf16 it is the correctly rounded value for every bf16 z in [-12, 12], where
+// tanh.approx is off by up to 1 % of it at z = -3 and all of it at z = -6.
+__device__ __forceinline__ float gelu_full(float z) {
+  const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
+  return __fdividef(z, 1.f + __expf(-2.f * u));
+}
+
 struct FwdParams {
   const __nv_bfloat16* x;    // [N][H][W][Cin]
   const __nv_bfloat16* w;    // [Cout][9][Cin]
@@ -209,7 +219,9 @@ __global__ void __launch_bounds__(NTH) k_conv3x3_fwd(const FwdParams p) {
         }
         if (p.z) *reinterpret_cast<__nv_bfloat162*>(p.z + o) = __floats2bfloat162_rn(v0, v1);
         if (p.a)
-          *reinterpret_cast<__nv_bfloat162*>(p.a + o) = __floats2bfloat162_rn(gelu(v0), gelu(v1));
+          *reinterpret_cast<__nv_bfloat162*>(p.a + o) =
+              p.z ? __floats2bfloat162_rn(gelu_full(v0), gelu_full(v1))
+                  : __floats2bfloat162_rn(gelu(v0), gelu(v1));
       }
     }
 }
@@ -687,7 +699,9 @@ __global__ void __launch_bounds__(160) k_conv3x3_fwd_tc(const FwdParams p) {
             v1 += __bfloat162float(r.y);
           }
           zz[e] = __floats2bfloat162_rn(v0, v1);
-          if (p.a) aa[e] = __floats2bfloat162_rn(gelu(v0), gelu(v1));
+          if (p.a)
+            aa[e] = p.z ? __floats2bfloat162_rn(gelu_full(v0), gelu_full(v1))
+                        : __floats2bfloat162_rn(gelu(v0), gelu(v1));
         }
         if (p.z) {
           reinterpret_cast<uint4*>(p.z + o)[0] = reinterpret_cast<const uint4*>(zz)[0];
@@ -997,7 +1011,9 @@ __global__ void __launch_bounds__(ST_NT) k_conv3x3_strip(const StripParams p) {
               v1 += __bfloat162float(rr.y);
             }
             zz[e] = __floats2bfloat162_rn(v0, v1);
-            if (p.a) aa[e] = __floats2bfloat162_rn(gelu(v0), gelu(v1));
+            if (p.a)
+              aa[e] = p.z ? __floats2bfloat162_rn(gelu_full(v0), gelu_full(v1))
+                          : __floats2bfloat162_rn(gelu(v0), gelu(v1));
           }
           if (p.z) {
             reinterpret_cast<uint4*>(p.z + o)[0] = reinterpret_cast<const uint4*>(zz)[0];

@@ -132,6 +132,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
       : "r"(addr));
 }
 
+// gelu_full() of two values
+__device__ __forceinline__ float2 gelu2_full(float2 z) {
+  const float k = -2.f * 0.7978845608028654f;
+  const float2 c = __ffma2_rn(__fmul2_rn(z, z), make_float2(k * 0.044715f, k * 0.044715f),
+                              make_float2(k, k));
+  const float2 u = __fmul2_rn(z, c);  // -2 u
+  const float2 d = __fadd2_rn(make_float2(__expf(u.x), __expf(u.y)), make_float2(1.f, 1.f));
+  return make_float2(__fdividef(z.x, d.x), __fdividef(z.y, d.y));
+}
+
 // A padded position: image, row and column of the (H + 2) x (W + 2) grid,
 // advanced by a fixed number of positions without divisions.
 struct PadPos {
@@ -167,7 +177,9 @@ struct FlowTile {
   static_assert(BN % 32 == 0 && BN <= 128 && MT % 2 == 0 && MT <= 8, "tile");
 };
 
-template <int BN, int MT, bool STREAM>
+// FULL: the activation by gelu_full (32 -> 32 channels, 16 x 256^2: 75.5 us, and
+// 67.8 with tanh.approx; with expf and a divide 109.5, most of it spills)
+template <int BN, int MT, bool STREAM, bool FULL>
 __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p) {
   using TT = FlowTile<BN, MT, STREAM>;
   constexpr int M = TT::M, ACC = TT::ACC, NBUF = TT::NBUF, CB = TT::CB, CH = TT::CH;
@@ -415,7 +427,7 @@ __global__ void __launch_bounds__(FL_NT, 1) k_conv3x3_flow(const FlowParams p) {
                 if (p.res) f = __fadd2_rn(f, f2bf(rr[hf].v[2 * e + i]));
                 if (p.z) zz.v[2 * e + i] = bf2(f.x, f.y);
                 if (p.a) {
-                  const float2 ge = gelu2(f);
+                  const float2 ge = FULL ? gelu2_full(f) : gelu2(f);
                   aa.v[2 * e + i] = bf2(ge.x, ge.y);
                 }
               }
@@ -456,15 +468,14 @@ int launch_flow(FlowParams p, cudaStream_t s) {
   p.S = flow_stages<BN, MT, STREAM>(p.cin, p.wid, &p.P);
   if (p.S == 0) return SP_EINVAL;
   const int smem = (STREAM ? 0 : 9 * p.cin * BN * 2) + p.S * (TT::CH * p.P * 16 + TT::WSTAGE) + 1024;
+  auto kern = p.z && p.a ? k_conv3x3_flow<BN, MT, STREAM, true> : k_conv3x3_flow<BN, MT, STREAM, false>;
   const cudaError_t attr =
-      cudaFuncSetAttribute(k_conv3x3_flow<BN, MT, STREAM>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (attr != cudaSuccess) return SP_ECUDA;
   const long long QN = (long long)(p.h + 2) * (p.wid + 2) * p.n;
   p.tiles = int((QN + TT::M - 1) / TT::M);
   const int ny = p.cout / BN, gx = sms() / ny > 0 ? sms() / ny : 1;
-  k_conv3x3_flow<BN, MT, STREAM><<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)),
-                                   FL_NT, smem, s>>>(p);
+  kern<<<dim3(unsigned(p.tiles < gx ? p.tiles : gx), unsigned(ny)), FL_NT, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ECUDA;
 }
 

@@ -122,3 +122,25 @@ def test_layer_autograd(skip):
     assert rel(layer.gw, wr.grad) < 4e-3 and rel(layer.gb, br.grad) < 8e-3
     if skip:
         assert rel(res.grad, rr.grad) < 4e-3
+
+
+@pytest.mark.parametrize("kernel", ["strip", "tc", "mma"])
+@pytest.mark.parametrize("co", [32, 128])
+def test_training_activation_is_rounded_once(kernel, co, monkeypatch):
+    """conv_gelu under autograd through a layer that copies its input (the centre
+    tap the identity, so that the pre-activation is every bf16 value in turn): the
+    activation is within half a unit in the last place of bf16 (2^-8 of the
+    value at most) and the 2^-20 that its fp32 arithmetic may add, also where 1 +
+    tanh cancels (down to fp32's smallest normal values, 12 / 2^126)."""
+    monkeypatch.setattr(S, "KERNEL", kernel)
+    v = torch.arange(0, 65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    v = v[(v.double().abs() <= 12) & (v.double().abs() >= 2.0 ** -20)].cuda()
+    v = torch.cat([v, v[: -v.numel() % (64 * co)]])
+    x = v.view(1, -1, 64, co).contiguous().requires_grad_()
+    layer = S.ConvLayer(co, co, torch.Generator().manual_seed(0))
+    layer.wb.zero_()
+    layer.wb[:, 1, 1, :] = torch.eye(co, device="cuda").bfloat16()
+    a = S.conv_gelu(x, layer).detach().double()
+    z = x.detach().double()
+    want = z / (1 + torch.exp(-2 * 0.7978845608028654 * (z + 0.044715 * z ** 3)))
+    assert ((a - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs() + 12 * 2.0 ** -126).all()
