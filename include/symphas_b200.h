@@ -292,7 +292,9 @@ int sp_conv3x3_fwd_strip_up2(const void* x, const void* w, void* wt, const float
                              int cout, void* stream);
 /* dw [cout][3][3][cin] (fp32) += weight gradient of that convolution for the
  * output gradient dy [n][h][w][cout]; cin a multiple of 32, cout of 8, fewer
- * than 2^31 pixels. */
+ * than 2^31 pixels.  For cout 32, 64 and multiples of 128 it runs on tcgen05:
+ * a CTA that gives up on a wait adds nothing, so that dw is then incomplete,
+ * and reports through sp_conv_tc_status. */
 int sp_conv3x3_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w_, int cin,
                      int cout, void* stream);
 /* x [npix][c] (bf16) = the fp32 field psi [npix] in channel 0 and zeros in

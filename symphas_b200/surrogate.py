@@ -77,6 +77,16 @@ def _fwd(x, wb, bias, res, z, a, ci, co, scratch=None):
                                    co, _s()), "sp_conv3x3_fwd")
 
 
+def check_waits():
+    """Raise if a tensor-memory kernel (a convolution or a weight gradient) gave
+    up on a wait since the last call: its output is then incomplete.  Waits for
+    the device."""
+    flag = ctypes.c_int(0)
+    _ok(C.lib().sp_conv_tc_status(ctypes.byref(flag)), "sp_conv_tc_status")
+    if flag.value:
+        raise C.SymPhasError(C.SP_ETIMEOUT, "a convolution gave up on a wait; its output is incomplete")
+
+
 class ConvLayer:
     """A 3x3 circular convolution: fp32 master weights [cout][3][3][cin] and
     bias, a bf16 copy for the kernels, gradient buffers and Adam moments."""
@@ -391,7 +401,8 @@ def train(net, snaps, steps=2000, batch=32, lr=1e-3, seed=0, log_every=200, log=
     scaled change): Adam with a linear warm-up over the first `warmup`
     fraction of the steps, cosine decay after it, and the gradients clipped to
     a global norm of `clip` (an occasional large batch gradient otherwise
-    throws the encoder-decoder off for good)."""
+    throws the encoder-decoder off for good).  Raises, where the loss is read,
+    if a kernel gave up on a wait (check_waits)."""
     ntraj, ns1, n, _ = snaps.shape
     pairs = ntraj * (ns1 - 1)
     d = snaps[:, 1:] - snaps[:, :-1]
@@ -424,6 +435,7 @@ def train(net, snaps, steps=2000, batch=32, lr=1e-3, seed=0, log_every=200, log=
         for l in layers:
             l.adam(step, lr_t)
         if step % log_every == 0 or step == steps:
+            check_waits()
             hist.append((step, float(loss.detach())))
             log("step %d loss %.4e (%.1f s)" % (step, hist[-1][1], time.perf_counter() - t0))
     return hist

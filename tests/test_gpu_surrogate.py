@@ -6,6 +6,7 @@ bit."""
 import pytest
 import torch
 
+from symphas_b200 import _capi as C
 from symphas_b200 import surrogate as S
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +77,18 @@ def test_trained_jump_reaches_t_end_faster_than_fd():
     assert ev["speedup"] > 1.2, ev
     assert ev["rel_l2_mean"] < 0.10, ev
     assert ev["max_mass_difference"] < 1e-4, ev
+
+
+def test_training_stops_where_a_kernel_gave_up(monkeypatch):
+    """A weight gradient that gave up is partial: training reads the flag where
+    it reads the loss."""
+    torch.cuda.set_device(0)
+    snaps = S.trajectories(2, 2, JUMP, N, DT, seed=3)
+
+    def gave_up(flag):
+        flag._obj.value = 1
+        return C.SP_OK
+
+    monkeypatch.setattr(C.lib(), "sp_conv_tc_status", gave_up)
+    with pytest.raises(C.SymPhasError):
+        S.train(S.JumpNet((32, 64)), snaps, steps=2, batch=2, log_every=1, log=lambda *_: None)

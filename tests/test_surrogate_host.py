@@ -3,6 +3,7 @@ pool, which redoes only the members the judge rejects on a model of about
 their count."""
 import pytest
 
+from symphas_b200 import _capi as C
 from symphas_b200 import surrogate as S
 
 
@@ -16,3 +17,23 @@ def test_fallback_pool_sizes(batch):
     for a, b in zip(sizes, sizes[1:]):
         assert b <= max(a + 1, int(a * 1.25 + 0.5)) or b == batch
     assert pool.models == {}  # nothing is created before it is needed
+
+
+class FakeLib:
+    """A library whose convolutions gave up `n` times since the last look."""
+
+    def __init__(self, n):
+        self.n = n
+
+    def sp_conv_tc_status(self, flag):
+        flag._obj.value, self.n = int(self.n > 0), 0
+        return C.SP_OK
+
+
+def test_check_waits_raises_once_for_a_kernel_that_gave_up(monkeypatch):
+    fake = FakeLib(2)
+    monkeypatch.setattr(C, "lib", lambda: fake)
+    with pytest.raises(C.SymPhasError) as e:
+        S.check_waits()
+    assert e.value.code == C.SP_ETIMEOUT
+    S.check_waits()
