@@ -850,6 +850,14 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   if (variant < 0 || variant >= int(H->variants.size()) || !applicable(H, variant)) variant = 0;
   if (int rc = configure(H, variant)) return rc;
   if (!getenv("SP_TILE")) many_plan(H, sp::find_many(key));
+  // constant sides hold their value from the start, whichever kernel steps first
+  // (the one-step kernels read the halo, the many-step kernel the description)
+  bool constant = false;
+  for (int s = 0; s < 2 * H->dim; ++s)
+    constant = constant || (dd.boundary[s] != SP_PERIODIC && dd.boundary_value[s] != 0.0);
+  for (int i = 0; constant && i < H->batch; ++i)
+    for (int f = 0; f < H->nf; ++f)
+      if (int rc = refresh_halos(H, i, f)) return rc;
   SP_CUDA(H, cudaDeviceSynchronize());
   return SP_OK;
 }

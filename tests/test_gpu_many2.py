@@ -125,3 +125,27 @@ def test_strip_step_on_ensembles(monkeypatch):
     for v in outs:
         for a, b in zip(outs[0], outs[v]):
             assert np.array_equal(a, b), v
+
+
+@pytest.mark.parametrize("dim,dims", [(2, (64, 48)), (2, (300, 200)), (3, (20, 16, 12))])
+@pytest.mark.parametrize("model,dtype,form", [("A", "f32", "fused"), ("C", "f64", "exact")])
+def test_constant_sides_before_the_first_upload(dim, dims, model, dtype, form):
+    """Steps from a handle's zero state: the same fields whether the steps come
+    in one call or one by one, and as after an upload of zeros."""
+    st = sp.Stencil2d2h(5, 6, 13) if dim == 2 else sp.Stencil3d2h(7, 10, 25)
+    params = sp.ProblemParameters(dims, boundary=WALLS["xy"],
+                                  boundary_value=[0.3, -0.2, 0.15, 0.05, 0.0, 0.0])
+    outs = []
+    for upload, chunks in ((True, (1,) * 6), (False, (1,) * 6), (False, (6,))):
+        m = MODELS[model](dim, sp.SolverFT(st, form=form), params, coeff=(0.8, 1.1), dtype=dtype,
+                          batch=2)
+        if upload:
+            for i in range(2):
+                for f in range(m.nfields):
+                    m.set_field(f, np.zeros(dims[::-1]), inst=i)
+        for s in chunks:
+            m.step(0.002, s)
+        outs.append(np.stack([m.get_field(f, inst=i) for i in range(2) for f in range(m.nfields)]))
+        m.close()
+    assert np.abs(outs[0]).max() > 0
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
