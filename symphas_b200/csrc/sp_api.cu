@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -700,17 +701,20 @@ void many_plan(sp_handle* H, const sp::ManyInfo* mi) {
     }
 }
 
-// fastest tile shape of each (kernel key, extents, batch) found so far
+// fastest tile shape of each (kernel key, extents, batch, periodic axes) found so
+// far: which shapes can run, and how they compare, depends on the sides
 std::mutex g_tune_mutex;
-std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int>, int> g_tuned;
+std::map<std::array<int, 12>, int> g_tuned;
 
 // the kernel-key code of a point count: 4th-order point sets are offset
 int pts_code(const sp_desc& d, int pts) { return d.accuracy == 4 ? sp::SP_PTS4 + pts : pts; }
 
-std::tuple<int, int, int, int, int, int, int, int, int, int, int> tune_key(const sp_handle* H) {
+std::array<int, 12> tune_key(const sp_handle* H) {
   const sp_desc& d = H->d;
+  int periodic = 0;
+  for (int a = 0; a < H->dim; ++a) periodic |= (d.boundary[2 * a] == SP_PERIODIC) << a;
   return {d.model, d.form, d.dim, d.dtype, pts_code(d, d.lap_pts), pts_code(d, d.gradlap_pts),
-          pts_code(d, d.bilap_pts), H->n[0], H->n[1], H->n[2], H->batch};
+          pts_code(d, d.bilap_pts), H->n[0], H->n[1], H->n[2], H->batch, periodic};
 }
 
 // kernel model of an ensemble: one model shared by every member, or the

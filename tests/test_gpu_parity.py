@@ -408,3 +408,28 @@ def test_row_kernels_on_a_batch_of_instances(cls, monkeypatch):
         rows += 1
     monkeypatch.delenv("SP_TILE")
     assert rows >= 1
+
+
+@pytest.mark.parametrize("model,dims", [(sp.model_MA_t, (128, 64, 48)), (sp.model_MB_t, (256, 40, 32)),
+                                        (sp.model_MC_t, (128, 48, 32))])
+def test_tuning_one_kind_of_sides_leaves_the_other(model, dims):
+    """A shape tuned on a grid periodic in x is not the starting shape of the
+    same grid with constant sides there, nor the other way round."""
+    P, D = sp.BoundaryType.PERIODIC, sp.BoundaryType.DEFAULT
+
+    def shape(walls, tune=False):
+        bc = [D, D, P, P, P, P] if walls else [P] * 6
+        m = model(3, sp.SolverFT(sp.Stencil3d2h(7, 10, 25), form="fused"),
+                  sp.ProblemParameters(dims, boundary=bc), dtype="f32")
+        if tune:
+            m.autotune(3)
+        v = m.kernel_info()["variant"]
+        m.close()
+        return v
+
+    walled, periodic = shape(True), shape(False)
+    tuned = shape(False, tune=True)
+    assert shape(True) == walled and shape(False) == tuned
+    tuned_walled = shape(True, tune=True)
+    assert shape(False) == tuned and shape(True) == tuned_walled
+    assert walled != periodic  # (a row kernel where x is periodic)
