@@ -704,7 +704,13 @@ void many_plan(sp_handle* H, const sp::ManyInfo* mi) {
 // fastest tile shape of each (kernel key, extents, batch, periodic axes) found so
 // far: which shapes can run, and how they compare, depends on the sides
 std::mutex g_tune_mutex;
-std::map<std::array<int, 12>, int> g_tuned;
+struct Tuned {
+  int variant;
+  // the many-step kernel against that shape: 1 taken (tile and depth), 0 not
+  // taken, -1 not timed
+  int many, many_tx, many_ty, many_kt;
+};
+std::map<std::array<int, 12>, Tuned> g_tuned;
 
 // the kernel-key code of a point count: 4th-order point sets are offset
 int pts_code(const sp_desc& d, int pts) { return d.accuracy == 4 ? sp::SP_PTS4 + pts : pts; }
@@ -834,7 +840,8 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   SP_CUDA(H, cudaMemset(H->err_d, 0, sizeof(int)));
 
   // tile shape: an explicit choice (SP_TILE), else the one sp_autotune found
-  // for this kernel and size in this process, else the first registered
+  // for this kernel and grid in this process (with its answer about the
+  // many-step kernel), else the preferred one
   int variant = 0;
   long long sites = 0;
   for (const InstGeo& g : H->geo) sites += g.sites();
@@ -845,15 +852,26 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
         sites >= k.pref_sites && filled <= k.pref_filled && applicable(H, v))
       variant = v;
   }
+  Tuned tuned{variant, -1, 0, 0, 0};
   if (!H->ensemble) {
     std::lock_guard<std::mutex> lk(g_tune_mutex);
     auto it = g_tuned.find(tune_key(H));
-    if (it != g_tuned.end()) variant = it->second;
+    if (it != g_tuned.end()) tuned = it->second;
+    variant = tuned.variant;
   }
   if (const char* t = getenv("SP_TILE")) variant = atoi(t);
   if (variant < 0 || variant >= int(H->variants.size()) || !applicable(H, variant)) variant = 0;
   if (int rc = configure(H, variant)) return rc;
-  if (!getenv("SP_TILE")) many_plan(H, sp::find_many(key));
+  if (!getenv("SP_TILE")) {
+    if (tuned.many < 0 || getenv("SP_MANY")) {
+      many_plan(H, sp::find_many(key));
+    } else if (tuned.many) {
+      H->many = sp::find_many(key);
+      H->many_tx = tuned.many_tx;
+      H->many_ty = tuned.many_ty;
+      H->many_kt = tuned.many_kt;
+    }
+  }
   // constant sides hold their value from the start, whichever kernel steps first
   // (the one-step kernels read the halo, the many-step kernel the description)
   bool constant = false;
@@ -1328,7 +1346,11 @@ int sp_autotune(sp_handle* H, int reps) {
   if ((rc = configure(H, best))) return rc;
   if (!H->ensemble) {
     std::lock_guard<std::mutex> lk(g_tune_mutex);
-    g_tuned[tune_key(H)] = best;
+    // (an answer that the environment forced is no answer for later handles)
+    const bool free = !getenv("SP_MANY") && !getenv("SP_TILE");
+    Tuned& t = g_tuned.emplace(tune_key(H), Tuned{best, -1, 0, 0, 0}).first->second;
+    t.variant = best;
+    if (many && free) t = {best, H->many != nullptr, H->many_tx, H->many_ty, H->many_kt};
   }
   return check_err_flag(H);
 }

@@ -149,3 +149,22 @@ def test_constant_sides_before_the_first_upload(dim, dims, model, dtype, form):
         m.close()
     assert np.abs(outs[0]).max() > 0
     assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("model,dims", [("A", (256, 256)), ("B", (804, 601)), ("B", (1024, 512)),
+                                        ("C", (640, 480)), ("A", (1024, 1024))])
+def test_later_handles_start_as_the_tuner_left_one(model, dims, monkeypatch):
+    """The tuner's answer about the many-step kernel, and not the estimate that
+    it may have overruled, is what later handles of the same grid start with."""
+    for k in ("SP_TILE", "SP_MANY"):
+        monkeypatch.delenv(k, raising=False)
+    got = []
+    for tune in (True, False):
+        m = MODELS[model](2, sp.SolverFT(sp.Stencil2d2h(5, 6, 13), form="fused"),
+                          sp.ProblemParameters(dims, boundary=[P] * 6), dtype="f32")
+        if tune:
+            m.autotune(5)
+        i = m.kernel_info()
+        got.append((i["variant"], i["steps_per_launch"]))
+        m.close()
+    assert got[0] == got[1]
