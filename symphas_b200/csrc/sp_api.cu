@@ -822,9 +822,8 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   H->plane = g0.plane;
   H->felems = g0.felems;
 
-  int dev = 0;
-  SP_CUDA(H, cudaGetDevice(&dev));
-  SP_CUDA(H, cudaDeviceGetAttribute(&H->sms, cudaDevAttrMultiProcessorCount, dev));
+  SP_CUDA(H, cudaGetDevice(&H->device));
+  SP_CUDA(H, cudaDeviceGetAttribute(&H->sms, cudaDevAttrMultiProcessorCount, H->device));
   SP_CUDA(H, cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking));
   H->own_stream = true;
 
@@ -915,18 +914,14 @@ cudaMemcpy3DParms interior_copy(sp_handle* H, int which, int inst, int field, vo
   return p;
 }
 
-// whether a kernel on this handle's device may read and write `p` as values:
-// plain device memory of the current device, aligned to the values (a copy
-// engine also takes what this refuses)
 bool kernel_copyable(const sp_handle* H, const void* p) {
   cudaPointerAttributes at{};
   int dev = -1;
-  if (reinterpret_cast<uintptr_t>(p) % H->esz != 0) return false;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return at.type == cudaMemoryTypeDevice && at.device == dev;
+  return copy_by_kernel(at, p, H->esz, dev, H->device);
 }
 
 // One instance's interior to or from device memory takes the copy kernel: an

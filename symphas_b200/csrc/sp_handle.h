@@ -6,6 +6,7 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <string>
 #include <vector>
@@ -48,6 +49,7 @@ struct sp_handle {
   int cur = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  int device = 0;  // the GPU of the buffers and the stream
   int sms = 148;
   // 3D grid
   int ntx = 1, nty = 1, nzc = 1, zchunk = 1;
@@ -81,6 +83,16 @@ struct sp_handle {
   double* cons_d = nullptr;  // [2] the latest reduction
   std::string err;
 };
+
+// Whether a kernel may move values between a field and a pointer of these
+// attributes: plain device memory of the handle's GPU, aligned to the values,
+// and that GPU current, since a kernel cannot be launched on the stream of
+// another (a copy engine takes all that this refuses).
+inline bool copy_by_kernel(const cudaPointerAttributes& at, const void* ptr, size_t esz, int current,
+                           int device) {
+  return reinterpret_cast<uintptr_t>(ptr) % esz == 0 && at.type == cudaMemoryTypeDevice &&
+         at.device == device && current == device;
+}
 
 // padded field `f` of instance `inst` in buffer `which`, and its interior origin
 inline char* field_base(sp_handle* H, int which, int inst, int f) {
