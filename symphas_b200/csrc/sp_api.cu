@@ -59,15 +59,16 @@ const ManyInfo* find_many(const KernelKey& key) {
   auto it = many_table().find(tup(key));
   return it == many_table().end() ? nullptr : &it->second;
 }
-// the built-in kernel sets (sp_inst_exact.cu, sp_inst_fused.cu,
-// sp_inst_wide.cu, sp_inst_many.cu, sp_inst_many_exact.cu); weak, so a program that compiles this runtime with only
-// its own models (the C++ front end, symphas_model.hpp) links without them
+// the built-in kernel sets (sp_inst_*.cu); weak, so a program that compiles
+// this runtime with only its own models (the C++ front end, symphas_model.hpp)
+// links without them
 void register_exact_kernels() __attribute__((weak));
 void register_fused_kernels() __attribute__((weak));
 void register_wide_kernels() __attribute__((weak));
 void register_exact3_kernels() __attribute__((weak));
 void register_many_kernels() __attribute__((weak));
 void register_many_exact_kernels() __attribute__((weak));
+void register_points_kernels() __attribute__((weak));
 void register_all_kernels() {
   static std::once_flag once;
   std::call_once(once, [] {
@@ -77,6 +78,7 @@ void register_all_kernels() {
     if (register_exact3_kernels) register_exact3_kernels();
     if (register_many_kernels) register_many_kernels();
     if (register_many_exact_kernels) register_many_exact_kernels();
+    if (register_points_kernels) register_points_kernels();
   });
 }
 

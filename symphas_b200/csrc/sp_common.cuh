@@ -128,6 +128,25 @@ __device__ __forceinline__ V fmadd(const V& a, const V& b, const V& c) {
   }
 }
 
+// a * b as a value of its own: under SP_EXPLICIT_FMA a product that no later sum
+// can absorb.  (ptxas fuses a packed multiply with a packed add that alone reads
+// it, __fmul2_rn and -fmad=false notwithstanding -- measured, 412 of 2048 sums --
+// and does not where another expression reads it too, so that two kernels of the
+// same expression may round differently; scalar products it leaves alone.)
+__device__ __forceinline__ float mul_own(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_own(double a, double b) { return __dmul_rn(a, b); }
+template <class V>
+__device__ __forceinline__ V rmul(const V& a, const V& b) {
+#ifdef SP_EXPLICIT_FMA
+  V r = a;
+#pragma unroll
+  for (int j = 0; j < int(sizeof(V) / sizeof(a.v[0])); ++j) r.v[j] = mul_own(a.v[j], b.v[j]);
+  return r;
+#else
+  return a * b;
+#endif
+}
+
 template <class T, int W>
 struct VecOf {
   using type = Vec<T, W>;

@@ -212,6 +212,15 @@ struct Reach<Gradlap<A>, ACC> : ReachD<A, ACC == 4 ? 3 : 2, ACC> {};
 template <class E>
 struct Ev;
 
+// r + the value of an operand; a product in it is not rounded on its own
+template <class A>
+struct Plus {
+  template <int X, int Y, int Z, class C, class V>
+  __device__ __forceinline__ static V at(const A& e, const C& c, const V& r) {
+    return r + Ev<A>::template at<X, Y, Z>(e, c);
+  }
+};
+
 template <class A, int X, int Y, int Z, class C>
 struct Shifted {
   const A& e;
@@ -219,6 +228,10 @@ struct Shifted {
   template <int i, int j, int k>
   __device__ __forceinline__ typename C::value_type at() const {
     return Ev<A>::template at<X + i, Y + j, Z + k>(e, c);
+  }
+  template <int i, int j, int k>
+  __device__ __forceinline__ typename C::value_type plus(const typename C::value_type& r) const {
+    return Plus<A>::template at<X + i, Y + j, Z + k>(e, c, r);
   }
 };
 
@@ -268,7 +281,7 @@ template <class A, class B>
 struct Ev<Mul<A, B>> {
   template <int X, int Y, int Z, class C>
   __device__ __forceinline__ static typename C::value_type at(const Mul<A, B>& e, const C& c) {
-    return Ev<A>::template at<X, Y, Z>(e.a, c) * Ev<B>::template at<X, Y, Z>(e.b, c);
+    return rmul(Ev<A>::template at<X, Y, Z>(e.a, c), Ev<B>::template at<X, Y, Z>(e.b, c));
   }
 };
 // a*b + c and its relatives: one FMA when the context may contract; in the
@@ -353,7 +366,30 @@ template <int N, class A>
 struct Ev<Pow<N, A>> {
   template <int X, int Y, int Z, class C>
   __device__ __forceinline__ static typename C::value_type at(const Pow<N, A>& e, const C& c) {
-    return rpow<N>(Ev<A>::template at<X, Y, Z>(e.a, c));
+    const typename C::value_type x = Ev<A>::template at<X, Y, Z>(e.a, c);
+    if constexpr (N == 1)
+      return x;
+    else
+      return rmul(x, rpow<N - 1>(x));
+  }
+};
+template <int N, class A>
+struct Plus<Pow<N, A>> {
+  template <int X, int Y, int Z, class C, class V>
+  __device__ __forceinline__ static V at(const Pow<N, A>& e, const C& c, const V& r) {
+    const V x = Ev<A>::template at<X, Y, Z>(e.a, c);
+    if constexpr (N == 1)
+      return r + x;
+    else
+      return fmadd<C::contract>(x, rpow<N - 1>(x), r);
+  }
+};
+template <class A, class B>
+struct Plus<Mul<A, B>> {
+  template <int X, int Y, int Z, class C, class V>
+  __device__ __forceinline__ static V at(const Mul<A, B>& e, const C& c, const V& r) {
+    return fmadd<C::contract>(Ev<A>::template at<X, Y, Z>(e.a, c),
+                              Ev<B>::template at<X, Y, Z>(e.b, c), r);
   }
 };
 template <class A>

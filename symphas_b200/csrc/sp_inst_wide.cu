@@ -81,8 +81,6 @@ void register_wide_kernels() {
   narrow3<MF_BMK_fused, 7>(SPK_BMK, 0.7, 400000, 0);
   tile<MF_C_fused, Tiles<float>::D3n1>(SPK_C, Pref{2, 1, 0, 1.0, 1500000});
   narrow3<MF_A_fused, 15>(SPK_A, 0.79, 400000, 1500000);
-  narrow3<MF_B_exact, 15>(SPK_B, 0.79, 400000, 1500000);
-  narrow3<MF_C_exact, 15>(SPK_C, 0.79, 400000, 1500000);
   // row kernels of the conserved pattern (x extent 256 or 128, periodic in x)
   row<EntryChRow<MF_B_fused, 256, 10, 1, 2, true, 2>>(SPK_B, 3);
   SP_REGCHROW(SPK_B, MF_B_fused, 256, 10, 1, 2, false, 2);

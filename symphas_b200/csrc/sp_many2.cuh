@@ -16,9 +16,9 @@
  * and sides may hold a constant: sites beyond such a side keep it in both
  * buffers, no step updates them, and staged operands are evaluated on them as
  * in the one-step kernels.  Sites are evaluated by the same expression code in
- * the same order, so s steps give the bits of s launches of k_fd2d (where a key
- * leaves the contraction of products to the compiler -- the fused form of
- * stencils other than <5,6,13> -- to its choice of roundings).
+ * the same order, so s steps give the bits of s launches of k_fd2d; keys whose
+ * products the compiler contracts as it sees fit have no many-step kernel
+ * (sp_inst_many_exact.cu) or spell the contractions out (sp_inst_points.cu).
  */
 #pragma once
 

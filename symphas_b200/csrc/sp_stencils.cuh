@@ -23,6 +23,10 @@ namespace sp {
 namespace st {
 
 #define K(x) T(x)
+// k v + r in one rounding, and r plus a point's value (SP_EXPLICIT_FMA: the point
+// sets of sp_inst_points.cu with their contractions spelled out)
+#define FM(k, v, r) fmadd<true>(T(k), v, r)
+#define PL(i, j, k, r) a.template plus<i, j, k>(r)
 #define P(i, j, k) a.template at<i, j, k>()
 #define v0 P(0, 0, 0)
 #define vx P(1, 0, 0)
@@ -153,7 +157,12 @@ template <> struct lap_pts<2, 5> {
 template <> struct lap_pts<2, 9> {
   template <class T, class A>
   __device__ __forceinline__ static T apply(const A& a, T divh2) {
+#ifdef SP_EXPLICIT_FMA
+    const T s = PL(-1, -1, 0, PL(1, 1, 0, PL(1, -1, 0, vx_y)));
+    return rmul(FM(-20., v0, FM(4., vx_, FM(4., vy_, FM(4., vy, FM(4., vx, s))))) * divh2, K(1.0 / 6));
+#else
     return (vx_y + vxy_ + vxy + vx_y_ + K(4.) * vx + K(4.) * vy + K(4.) * vy_ + K(4.) * vx_ - K(20.) * v0) * divh2 * K(1.0 / 6);
+#endif
   }
 };
 template <> struct lap_pts<3, 7> {
@@ -165,7 +174,14 @@ template <> struct lap_pts<3, 7> {
 template <> struct lap_pts<3, 15> {
   template <class T, class A>
   __device__ __forceinline__ static T apply(const A& a, T divh2) {
+#ifdef SP_EXPLICIT_FMA
+    T s = PL(1, 1, -1, PL(-1, 1, -1, PL(1, -1, -1, vx_y_z_)));
+    s = PL(1, 1, 1, PL(-1, 1, 1, PL(1, -1, 1, PL(-1, -1, 1, s))));
+    const T f = PL(0, 0, -1, PL(0, 0, 1, PL(0, -1, 0, PL(0, 1, 0, PL(1, 0, 0, vx_)))));
+    return rmul(FM(8., FM(-7., v0, f), s) * divh2, K(1.0 / 12));
+#else
     return (vx_y_z_ + vxy_z_ + vx_yz_ + vxyz_ + vx_y_z + vxy_z + vx_yz + vxyz + K(8.) * (vx_ + vx + vy + vy_ + vz + vz_ - K(7.) * v0)) * divh2 * K(1.0 / 12);
+#endif
   }
 };
 template <> struct lap_pts<3, 19> {
@@ -191,7 +207,11 @@ template <int DIM, int N> struct bilap_pts;
 template <> struct bilap_pts<2, 13> {
   template <class T, class A>
   __device__ __forceinline__ static T apply(const A& a, T divh4) {
+#ifdef SP_EXPLICIT_FMA
+    return rmul(FM(20., v0, FM(-8., vx_ + vx + vy_ + vy, FM(2., vx_y_ + vxy_ + vx_y + vxy, vy2_ + vy2 + vx2_ + vx2))), divh4);
+#else
     return (vy2_ + vy2 + vx2_ + vx2 + K(2.) * (vx_y_ + vxy_ + vx_y + vxy) - K(8.) * (vx_ + vx + vy_ + vy) + K(20.) * v0) * divh4;
+#endif
   }
 };
 template <> struct bilap_pts<2, 17> {
@@ -215,7 +235,12 @@ template <> struct bilap_pts<3, 21> {
 template <> struct bilap_pts<3, 25> {
   template <class T, class A>
   __device__ __forceinline__ static T apply(const A& a, T divh4) {
+#ifdef SP_EXPLICIT_FMA
+    const T far = vx2 + vx2_ + vy2 + vy2_ + vz2 + vz2_, near = vx + vx_ + vy + vy_ + vz + vz_;
+    return rmul(FM(42., v0, FM(-12., near, FM(2., vxy + vx_y + vxy_ + vx_y_ + vxz_ + vx_z_ + vxz + vx_z + vyz_ + vyz + vy_z_ + vy_z, far))), divh4);
+#else
     return (K(2.) * (vxy + vx_y + vxy_ + vx_y_ + vxz_ + vx_z_ + vxz + vx_z + vyz_ + vyz + vy_z_ + vy_z) + (vx2 + vx2_ + vy2 + vy2_ + vz2 + vz2_) - K(12.) * (vx + vx_ + vy + vy_ + vz + vz_) + K(42.) * v0) * divh4;
+#endif
   }
 };
 template <> struct bilap_pts<3, 41> {

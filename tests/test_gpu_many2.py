@@ -168,3 +168,18 @@ def test_later_handles_start_as_the_tuner_left_one(model, dims, monkeypatch):
         got.append((i["variant"], i["steps_per_launch"]))
         m.close()
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("model", sorted(MODELS))
+@pytest.mark.parametrize("dtype,form,wide", [("f32", "fused", True), ("f64", "fused", True),
+                                             ("f32", "exact", True), ("f32", "exact", False),
+                                             ("f64", "exact", True), ("f32", "fused", False)])
+@pytest.mark.parametrize("dims,walls", [((64, 64), ""), ((101, 53), "x"), ((300, 200), "")])
+def test_bits_do_not_depend_on_the_calls(model, dtype, form, wide, dims, walls, monkeypatch):
+    """A run in one call, in single steps and in uneven calls: the same bits, on
+    every point set of the dispatch."""
+    if wide and form == "fused" and model in ("AMK", "BMK"):
+        pytest.skip("no such kernel")
+    outs = [run(monkeypatch, {}, model, dims, dtype, form, 0, walls, wide=wide, chunks=c)[0]
+            for c in ((25,), (1,) * 25, (7, 1, 13, 4))]
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
