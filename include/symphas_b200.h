@@ -324,6 +324,13 @@ int sp_conv3x3_out1(const void* x, const void* w, const float* bias, float* out,
  * 8; z, da, dz 16-byte aligned.  No counterpart in SymPhas. */
 int sp_gelu_bwd_bf16(const void* z, const void* da, void* dz, float* db, long long npix, int c,
                      void* stream);
+/* The same with the sums taken in a fixed order, so that equal inputs give equal
+ * bits of db (sp_gelu_bwd_bf16 adds them as the CTAs end): `scratch` is device
+ * memory of the floats that sp_gelu_bwd_scratch returns for this GPU, free again
+ * when the call's work on the stream is done.  No counterpart in SymPhas. */
+int sp_gelu_bwd_scratch(long long npix, int c, long long* floats);
+int sp_gelu_bwd_ordered_bf16(const void* z, const void* da, void* dz, float* db, float* scratch,
+                             long long npix, int c, void* stream);
 /* wf [cin][3][3][cout] = w [cout][3][3][cin] rotated by 180 degrees: the input
  * gradient of the convolution is sp_conv3x3_fwd(dy, wf). */
 int sp_conv3x3_flip(const void* w, void* wf, int cin, int cout, void* stream);

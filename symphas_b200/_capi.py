@@ -137,6 +137,10 @@ SIGNATURES = {
     "sp_conv3x3_out1": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                        ctypes.c_int, _P]),
     "sp_gelu_bwd_bf16": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_longlong, ctypes.c_int, _P]),
+    "sp_gelu_bwd_scratch": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_int,
+                                           ctypes.POINTER(ctypes.c_longlong)]),
+    "sp_gelu_bwd_ordered_bf16": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_longlong,
+                                                ctypes.c_int, _P]),
     "sp_conv3x3_wgrad": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                         ctypes.c_int, ctypes.c_int, _P]),
     "sp_conv3x3_flip": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int, _P]),

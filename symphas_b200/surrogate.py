@@ -143,8 +143,7 @@ class _Conv(torch.autograd.Function):
         (x,) = ctx.saved_tensors
         L = ctx.layer
         dz = _aligned(dz)
-        _ok(C.lib().sp_gelu_bwd_bf16(None, _p(dz), None, _p(L.gb), dz.numel() // L.cout, L.cout,
-                                     _s()), "sp_gelu_bwd_bf16")
+        _act_grad(None, dz, None, L)
         dx = _grads(x, dz, L, ctx.needs_input_grad[0])
         return dx, None, None, (dz if ctx.has_res else None)
 
@@ -153,6 +152,16 @@ def _aligned(g):
     """A gradient as the kernels read it: contiguous bf16 on a 16-byte boundary."""
     g = g.contiguous().bfloat16()
     return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
+def _act_grad(z, da, dz, L):
+    """dz = da * gelu'(z) (none with z None), and its bias gradient accumulated in
+    the layer, summed in a fixed order."""
+    npix, need = da.numel() // L.cout, ctypes.c_longlong()
+    _ok(C.lib().sp_gelu_bwd_scratch(npix, L.cout, ctypes.byref(need)), "sp_gelu_bwd_scratch")
+    scratch = torch.empty(need.value, device="cuda")
+    _ok(C.lib().sp_gelu_bwd_ordered_bf16(_p(z), _p(da), _p(dz), _p(L.gb), _p(scratch), npix, L.cout,
+                                         _s()), "sp_gelu_bwd_ordered_bf16")
 
 
 def _grads(x, dz, L, need_dx):
@@ -191,8 +200,7 @@ class _ConvGelu(torch.autograd.Function):
         L = ctx.layer
         da = _aligned(da)
         dz = torch.empty_like(z)
-        _ok(C.lib().sp_gelu_bwd_bf16(_p(z), _p(da), _p(dz), _p(L.gb), z.numel() // L.cout, L.cout,
-                                     _s()), "sp_gelu_bwd_bf16")
+        _act_grad(z, da, dz, L)
         dx = _grads(x, dz, L, ctx.needs_input_grad[0])
         return dx, None, None, (dz if ctx.has_res else None)
 

@@ -144,3 +144,43 @@ def test_training_activation_is_rounded_once(kernel, co, monkeypatch):
     z = x.detach().double()
     want = z / (1 + torch.exp(-2 * 0.7978845608028654 * (z + 0.044715 * z ** 3)))
     assert ((a - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs() + 12 * 2.0 ** -126).all()
+
+
+@pytest.mark.parametrize("npix,c", [(1, 8), (7, 24), (1000, 32), (33, 256), (9, 2056), (300000, 64)])
+@pytest.mark.parametrize("with_z", [False, True])
+def test_ordered_bias_gradient(npix, c, with_z):
+    """The same bits in every run, and the sums of dz as stored."""
+    torch.manual_seed(c)
+    z = (3 * torch.randn(npix, c, device="cuda")).bfloat16() if with_z else None
+    da = torch.randn(npix, c, device="cuda").bfloat16()
+    dz = torch.empty_like(da) if with_z else None
+    need = ctypes.c_longlong()
+    assert C.lib().sp_gelu_bwd_scratch(npix, c, ctypes.byref(need)) == C.SP_OK
+    got = []
+    for _ in range(8):
+        db = torch.ones(c, device="cuda")
+        ws = torch.full((need.value + 1,), float("nan"), device="cuda")
+        assert C.lib().sp_gelu_bwd_ordered_bf16(ptr(z), ptr(da), ptr(dz), ptr(db), ptr(ws), npix, c,
+                                                stream()) == C.SP_OK
+        assert torch.isnan(ws[-1])
+        got.append(db)
+    assert all(torch.equal(got[0], g) for g in got)
+    v = (dz if with_z else da).double()
+    bound = npix * 2.0 ** -24 * (v.abs().sum(0) + 1) + 1e-6
+    assert ((got[0].double() - 1 - v.sum(0)).abs() <= bound).all()
+    assert C.lib().sp_gelu_bwd_ordered_bf16(ptr(z), ptr(da), ptr(dz), ptr(got[0]), None, npix, c,
+                                            stream()) == C.SP_EINVAL
+
+
+def test_layer_bias_gradient_repeats_itself():
+    torch.manual_seed(9)
+    n, h, w, ci, co = 8, 96, 96, 32, 64
+    layer = S.ConvLayer(ci, co, torch.Generator().manual_seed(1))
+    x = torch.randn(n, h, w, ci, device="cuda").bfloat16()
+    dy = torch.randn(n, h, w, co, device="cuda").bfloat16()
+    got = []
+    for _ in range(6):
+        layer.zero_grad()
+        S.conv_gelu(x, layer).backward(dy)
+        got.append(layer.gb.clone())
+    assert all(torch.equal(got[0], g) for g in got)
