@@ -433,3 +433,39 @@ def test_tuning_one_kind_of_sides_leaves_the_other(model, dims):
     tuned_walled = shape(True, tune=True)
     assert shape(False) == tuned and shape(True) == tuned_walled
     assert walled != periodic  # (a row kernel where x is periodic)
+
+
+MC, MAMK, MBMK = sp.model_MC_t, sp.model_MAMK_t, sp.model_MBMK_t
+
+
+@pytest.mark.parametrize("dims", [(36, 22, 18), (75, 20, 15), (128, 12, 10)])
+@pytest.mark.parametrize("cls,dtype,form,wide", [
+    (sp.model_MA_t, "f32", "fused", True), (sp.model_MB_t, "f32", "fused", True),
+    (MC, "f32", "fused", True), (MAMK, "f32", "fused", False), (MBMK, "f32", "fused", False),
+    (sp.model_MA_t, "f64", "exact", False), (MAMK, "f64", "exact", False),
+    (sp.model_MB_t, "f64", "exact", False), (MC, "f64", "exact", False),
+    (MBMK, "f64", "exact", False)])
+def test_shapes_of_every_3d_key_give_the_same_fields(cls, dtype, form, wide, dims, monkeypatch):
+    """Every tile shape of the 15-point forms, of AMK and BMK and of the exact
+    FP64 models against the first one, on extents that tiles do not divide, with
+    constant sides in y."""
+    P, D = sp.BoundaryType.PERIODIC, sp.BoundaryType.DEFAULT
+    ref, ran = None, 0
+    for v in range(64):
+        monkeypatch.setenv("SP_TILE", str(v))
+        m = cls(3, sp.SolverFT(sp.Stencil3d2h() if wide else sp.Stencil3d2h(7, 10, 25), form=form),
+                sp.ProblemParameters(dims, boundary=[P, P, D, D, P, P], boundary_value=0.2),
+                coeff=(0.8, 1.1), dtype=dtype)
+        if v >= m.kernel_info()["variants"]:
+            m.close()
+            break
+        if m.kernel_info()["variant"] == v:
+            for f in range(m.nfields):
+                m.fill_uniform(f, 60 + f, -0.3, 0.1)
+            m.step(0.004, 5)
+            out = np.stack([m.get_field(f) for f in range(m.nfields)])
+            ref = out if ref is None else ref
+            assert np.array_equal(out, ref), v
+            ran += 1
+        m.close()
+    assert ran > 1

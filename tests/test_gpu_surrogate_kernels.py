@@ -80,7 +80,7 @@ def test_conv_input_and_weight_gradients():
 
 
 def test_weight_gradient_many_chunks():
-    """Enough pixels that the split-K grid has many chunks per tile."""
+    """Pixels split over many CTAs, whose sums are all added into dw."""
     torch.manual_seed(2)
     n, h, w, ci, co = 4, 64, 64, 64, 32
     x = torch.randn(n, h, w, ci, device="cuda").bfloat16()
@@ -113,3 +113,25 @@ def test_adam_matches_the_update_rule():
     torch.cuda.synchronize()
     assert torch.allclose(w, ref_w, rtol=1e-5, atol=1e-6)
     assert torch.equal(wb, w.bfloat16())
+
+
+@pytest.mark.parametrize("n,h,w,ci,co", [(1, 3, 5, 32, 8), (2, 9, 11, 64, 40), (4, 64, 64, 32, 96),
+                                         (3, 33, 47, 96, 72), (1, 40, 100, 32, 200)])
+def test_weight_gradient_on_mma_sync(n, h, w, ci, co):
+    """Output channels outside 32, 64 and multiples of 128 keep the mma.sync
+    kernel: a partial block of 64 columns, fewer pixels than a chunk and several
+    split-K chunks, a last chunk that is not full; on top of what dw holds."""
+    torch.manual_seed(co)
+    x = torch.randn(n, h, w, ci, device="cuda").bfloat16()
+    dy = torch.randn(n, h, w, co, device="cuda").bfloat16()
+    base = torch.randn(co, 3, 3, ci, device="cuda")
+    dw = base.clone()
+    assert C.lib().sp_conv3x3_wgrad(ptr(x), ptr(dy), ptr(dw), n, h, w, ci, co,
+                                    stream()) == C.SP_OK
+    d = dy.double().reshape(-1, co)
+    want = torch.empty(co, 3, 3, ci, device="cuda", dtype=torch.float64)
+    for t in range(9):
+        xs = torch.roll(x.double(), (1 - t // 3, 1 - t % 3), (1, 2)).reshape(-1, ci)
+        want[:, t // 3, t % 3] = d.t() @ xs
+    # fp32 sums of at most 16384 products, plus the accumulation into dw
+    assert float((dw.double() - base.double() - want).abs().max() / want.abs().max()) < 1e-4
