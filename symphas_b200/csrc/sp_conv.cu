@@ -1159,8 +1159,11 @@ int strip_fwd(const void* x, const void* w, void* wt, const float* bias, const v
     if (rc != SP_EINVAL) return rc;
   }
   const int bn = cout == 32 ? 32 : cout == 64 ? 64 : 128;
-  // CTA shape by layer class, from timing every shape on the jump network's
-  // layers (256 samples, 256^2 .. 32^2): narrow outputs gain from more,
+  // What is left here: weights or a residual off 16 bytes, cin % 32 == 16 with 32
+  // or 64 outputs, and strips that do not fit beside resident weights.  CTA shape
+  // by layer class, from timing every shape on the jump network's layers (256
+  // samples, 256^2 .. 32^2), before those that fit moved to the persistent
+  // kernel: narrow outputs gain from more,
   // smaller CTAs (four or two M-tiles, one stage, so that more CTAs share an
   // SM and one CTA's gather overlaps another's MMAs and epilogue); wide
   // inputs and outputs keep the four-stage ring of 32-channel K blocks

@@ -28,7 +28,6 @@ import time
 
 import numpy as np
 import torch
-import torch.nn.functional as F
 
 from . import _capi as C
 from .model import ProblemParameters, SolverFT, Stencil2d2h, model_MB_t
@@ -207,10 +206,6 @@ class _ConvGelu(torch.autograd.Function):
 
 def conv(x, layer, res=None):
     return _Conv.apply(x, layer.anchor, layer, res)
-
-
-def gelu(z):
-    return F.gelu(z, approximate="tanh")
 
 
 def conv_gelu(x, layer, res=None):
