@@ -99,7 +99,8 @@ typedef struct sp_desc {
 typedef struct sp_handle sp_handle;
 
 /* Create a handle: validates the description, allocates the device fields
- * (interior + halo, ping-pong) and builds the TMA descriptors. */
+ * (interior + halo, ping-pong) and builds the TMA descriptors.  The fields start
+ * at zero, with the constants of their sides around them. */
 int sp_create(const sp_desc* desc, sp_handle** out);
 
 /* ---- ensembles of independent 2D systems --------------------------------
@@ -274,9 +275,12 @@ int sp_conv_tc_status(int* gave_up);
  * memory (the CTA shape is chosen per layer class; SP_STRIP_SHAPE="mt,cb,s"
  * fixes it for timing),
  * the weights re-tiled into `wt` (9 cin cout bf16 of scratch, device memory)
- * and loaded with one bulk copy per channel block.  Where the weights and two
- * strips fit in shared memory (cin a multiple of 32) a persistent kernel with
- * resident weights runs instead and leaves `wt` alone.  cin a multiple of 16,
+ * and loaded with one bulk copy per channel block.  Where w and res start on 16
+ * bytes a persistent kernel runs instead: with resident weights, and `wt` left
+ * alone, where they and two strips fit in shared memory (cin a multiple of 32);
+ * else, for cout a multiple of 128, with the weights re-tiled into `wt` and
+ * streamed.  `wt` may thus be written by every call: calls that can overlap need
+ * one each.  cin a multiple of 16,
  * cout 32, 64 or a multiple of 128, w_ <= 764; x, wt, bias, z and a 16-byte
  * aligned, res on 4 bytes, w any (w or res off 16 bytes keep the strip
  * kernel); bounded waits report through sp_conv_tc_status. */

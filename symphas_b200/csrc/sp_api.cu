@@ -680,7 +680,7 @@ void many_plan(sp_handle* H, const sp::ManyInfo* mi) {
       const int ty = (n1 + gy - 1) / gy;
       // the same columns with fewer rows of tiles cannot be better: about 20
       // candidates a depth instead of 148 (every sp_create pays for this loop:
-      // 64^2, 48 us on the host with all of them, 11 so)
+      // 64^2, 48 us on the host with all of them, 4 so)
       if (tx == last) continue;
       last = tx;
       if (!fits(tx, ty, kt)) continue;

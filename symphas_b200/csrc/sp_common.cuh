@@ -59,7 +59,8 @@ __device__ __forceinline__ Vec<T, W> operator-(const Vec<T, W>& a) {
 // Two FP32 lanes map onto Blackwell's packed FP32x2 instructions
 // (__fadd2_rn / __fmul2_rn / __ffma2_rn, sm_100): one instruction per two
 // sites, each lane rounded exactly as the scalar operation (a - b is
-// a + (-b), which is exact).
+// a + (-b), which is exact), except that ptxas may fuse a product with the one
+// sum that reads it (rmul below).
 __device__ __forceinline__ float2 f2(const Vec<float, 2>& a) { return make_float2(a.v[0], a.v[1]); }
 __device__ __forceinline__ Vec<float, 2> v2(float2 a) {
   Vec<float, 2> r;

@@ -1,6 +1,7 @@
 /*
  * sp_flow.cuh -- the 3x3 circular convolution (forward and data gradient) as a
- * persistent tcgen05 kernel with the weights resident in shared memory.  No
+ * persistent tcgen05 kernel, with the weights resident in shared memory, or, for
+ * 128 outputs and more where they do not fit, streamed with the input.  No
  * counterpart in SymPhas.
  *
  * Same operand layout as k_conv3x3_strip (sp_conv.cu): the input is staged as
@@ -8,9 +9,10 @@
  * position and 8-channel chunk), so the nine taps are nine start addresses of
  * one staged strip.  What differs:
  *
- *   - one CTA per SM walks over the tiles (MT x 128 positions each); the
+ *   - one CTA per SM walks over the tiles (MT x 128 positions each); resident
  *     weights of its BN output channels are gathered once per CTA, straight
- *     from [cout][3][3][cin] (no re-tiling launch);
+ *     from [cout][3][3][cin] (no re-tiling launch); streamed ones are re-tiled by
+ *     k_tile_weights and come with every stage;
  *   - gather, MMAs and epilogue of different tiles overlap: eight producer
  *     warps fill a ring of strips (32 input channels each), one thread issues
  *     the MMAs into one of two tensor-memory accumulators, sixteen warps empty

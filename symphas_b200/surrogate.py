@@ -50,12 +50,14 @@ def _ok(rc, what):
 
 # The forward convolutions (and the data gradients, forward convolutions of
 # the flipped weights) run on
-#   "strip"  the tcgen05 kernel that stages each input pixel once and reads the
-#            nine taps as operand offsets (sp_conv3x3_fwd_strip), where its
+#   "strip"  the tcgen05 kernels that stage each input pixel once and read the
+#            nine taps as operand offsets (sp_conv3x3_fwd_strip), where their
 #            shapes allow (cin % 16 == 0, cout 32, 64 or a multiple of 128,
 #            width <= 764), else on the next;
 #   "tc"     the tcgen05 kernel with a per-tap gather (sp_conv3x3_fwd_tc);
 #   "mma"    the mma.sync kernel (sp_conv3x3_fwd).
+# The network's first and last layer at inference have kernels of their own,
+# whatever it says.
 KERNEL = "strip"
 
 
