@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(TC::NT)
   // output rows of this thread
   const int x = x0 + txt * W;
   const bool xin = x < p.n[0];
-  const bool vec_ok = (p.n[0] % W == 0) && (x + W <= p.n[0]);
+  const bool vec_ok = whole_groups<W, R>(p.n[0]) && (x + W <= p.n[0]);
   const long long xo = image_offset(p.per[0], x, W, p.n[0], R, 1);
   T* orow[SPT];
   bool rowin[SPT];

@@ -116,6 +116,16 @@ struct HaloGeom {
                                      imax(16 / (int)sizeof(T), W));
 };
 
+// Whether rows of n0 sites are stored in whole W-groups: n0 is a multiple of W,
+// and no group lies within the reach R of both periodic faces (a group has one
+// image along x; on rows of one or two groups it would need two, and goes element
+// by element).  No extent is below 4, so only W = 4 and R = 3 ask.
+template <int W, int R>
+__device__ __forceinline__ bool whole_groups(int n0) {
+  constexpr int from = R > 0 ? (R - 1) / W * W + W + R : 0;
+  return n0 % W == 0 && (from <= 4 || n0 >= from);
+}
+
 // Store the W values of one site group at interior (x, y, z) (x a multiple of
 // W).  Interior groups take one vector store; groups within the stencil reach
 // of a periodic face also store their images into the halo, element by element.
@@ -123,7 +133,7 @@ template <class T, int W, int DIM, int R>
 __device__ __forceinline__ void store_group(T* org, int x, int y, int z, const vec_t<T, W>& v,
                                             const int* n, const int* h, const int* per,
                                             long long pitch, long long plane) {
-  if (x + W <= n[0] && n[0] % W == 0) {
+  if (x + W <= n[0] && whole_groups<W, R>(n[0])) {
     // whole group: it and each of its periodic images is one vector store
     int xs[2] = {x + h[0], 0}, ys[2] = {y + h[1], 0}, zs[2] = {DIM == 3 ? z + h[2] : 0, 0};
     int cx = 1, cy = 1, cz = 1;
@@ -384,7 +394,7 @@ __global__ void __launch_bounds__(TC::NT)
   const bool xin = x < p.n[0];
   // whole W-groups (every group but a ragged row end) store as vectors, their
   // periodic images too
-  const bool vec_ok = (p.n[0] % W == 0) && (x + W <= p.n[0]);
+  const bool vec_ok = whole_groups<W, R>(p.n[0]) && (x + W <= p.n[0]);
   const long long xo = image_offset(p.per[0], x, W, p.n[0], R, 1);
   T* orow[SPT][NF];
   bool rowin[SPT];
@@ -760,7 +770,7 @@ __device__ __forceinline__ void fd2_out(const Step2Params<T>& p, const M& m, con
       nv[k][1] = p.rhs_only ? r1 : fmadd<!K::exact>(vdt, r1, ctx.template var<2, 0, 0, 0>());
     }
   }
-  const bool vec_ok = (n0 % W == 0) && (x + W <= n0);
+  const bool vec_ok = whole_groups<W, R>(n0) && (x + W <= n0);
   const long long xo = image_offset(ip.per[0], x, W, n0, R, 1);
   const int h[3] = {p.hx, p.hy, 0};
   const int n3[3] = {n0, n1, 1};

@@ -469,3 +469,47 @@ def test_shapes_of_every_3d_key_give_the_same_fields(cls, dtype, form, wide, dim
             ran += 1
         m.close()
     assert ran > 1
+
+
+@pytest.mark.parametrize("dims", [(4, 20, 12), (4, 9, 33), (5, 8, 6), (8, 12, 9), (4, 24), (6, 40)])
+@pytest.mark.parametrize("cls", [sp.model_MA_t, sp.model_MB_t, MC, MAMK, MBMK])
+def test_rows_of_one_group_are_periodic(cls, dims, monkeypatch):
+    """Rows so short that a group of four sites lies at both periodic faces:
+    the library's own choice and every shape against the FP64 one."""
+    dim = len(dims)
+    st = S2 if dim == 2 else S3
+    want, ran = None, 0
+    for v, dtype in [("0", "f64"), (None, "f32")] + [(str(k), "f32") for k in range(40)]:
+        monkeypatch.delenv("SP_TILE", raising=False)
+        if v is not None:
+            monkeypatch.setenv("SP_TILE", v)
+        m = cls(dim, sp.SolverFT(st, form="fused"), sp.ProblemParameters(dims), coeff=(0.8, 1.1),
+                dtype=dtype)
+        if v is None or m.kernel_info()["variant"] == int(v):
+            for f in range(m.nfields):
+                m.fill_uniform(f, 5 + f, -0.3, 0.1)
+            m.step(0.004, 8)
+            out = np.stack([m.get_field(f) for f in range(m.nfields)])
+            want = out if want is None else want
+            # eight steps in FP32 on fields of 0.3 at most: some 2^-24 a step
+            assert np.abs(out - want).max() <= 1e-5, v
+            ran += 1
+        m.close()
+    assert ran > 2
+
+
+@pytest.mark.parametrize("form", ["exact", "fused"])
+@pytest.mark.parametrize("dims", [(6, 17), (7, 12), (8, 9)])
+def test_fourth_order_rows_near_twice_the_reach(form, dims):
+    """4th-order stencils reach three sites: on rows of six a group of two is at
+    both faces.  The fields of the transposed grid, whose rows are long."""
+    outs = []
+    for d in (dims, dims[::-1]):
+        x = np.random.default_rng(2).uniform(-0.3, 0.1, dims[::-1])
+        m = sp.model_MB_t(2, sp.SolverFT(sp.Stencil2d4h(), form=form), sp.ProblemParameters(d),
+                          dtype="f64")
+        m.set_field(0, x if d == dims else x.T.copy())
+        m.step(0.002, 9)
+        outs.append(m.get_field(0))
+        m.close()
+    assert np.abs(outs[0] - outs[1].T).max() <= 1e-13
