@@ -65,6 +65,14 @@ def _strip_ok(ci, co, w):
     return ci % 16 == 0 and (co in (32, 64) or co % 128 == 0) and w <= 764
 
 
+def _dense(t):
+    """A tensor as the kernels read it: contiguous, on a 16-byte boundary."""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _fwd(x, wb, bias, res, z, a, ci, co, scratch=None):
     n, h, w = x.shape[:3]
     if KERNEL == "strip" and scratch is not None and _strip_ok(ci, co, w):
@@ -131,6 +139,7 @@ class _Conv(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, anchor, layer, res):
+        x, res = _dense(x), _dense(res)
         n, h, w, ci = x.shape
         z = torch.empty(n, h, w, layer.cout, device="cuda", dtype=torch.bfloat16)
         _fwd(x, layer.wb, layer.b, res, z, None, ci, layer.cout, layer.wt)
@@ -150,9 +159,8 @@ class _Conv(torch.autograd.Function):
 
 
 def _aligned(g):
-    """A gradient as the kernels read it: contiguous bf16 on a 16-byte boundary."""
-    g = g.contiguous().bfloat16()
-    return g if g.data_ptr() % 16 == 0 else g.clone()
+    """A gradient as the kernels read it: in bf16, contiguous, on 16 bytes."""
+    return _dense(g.bfloat16())
 
 
 def _act_grad(z, da, dz, L):
@@ -186,6 +194,7 @@ class _ConvGelu(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, anchor, layer, res):
+        x, res = _dense(x), _dense(res)
         n, h, w, ci = x.shape
         z = torch.empty(n, h, w, layer.cout, device="cuda", dtype=torch.bfloat16)
         a = torch.empty_like(z)
@@ -215,6 +224,7 @@ def conv_gelu(x, layer, res=None):
     epilogue; without autograd no pre-activation is kept."""
     if torch.is_grad_enabled():
         return _ConvGelu.apply(x, layer.anchor, layer, res)
+    x, res = _dense(x), _dense(res)
     n, h, w, ci = x.shape
     a = torch.empty(n, h, w, layer.cout, device="cuda", dtype=torch.bfloat16)
     _fwd(x, layer.wb, layer.b, res, None, a, ci, layer.cout, layer.wt)
@@ -228,8 +238,9 @@ def conv_gelu_up(x, layer, res=None):
     n, h, w, ci = x.shape
     if torch.is_grad_enabled() or KERNEL != "strip" or not _strip_ok(ci, layer.cout, 2 * w):
         return conv_gelu(up2(x), layer, res)
+    x, res = _dense(x), _dense(res)
     a = torch.empty(n, 2 * h, 2 * w, layer.cout, device="cuda", dtype=torch.bfloat16)
-    _ok(C.lib().sp_conv3x3_fwd_strip_up2(_p(x.contiguous()), _p(layer.wb), _p(layer.wt),
+    _ok(C.lib().sp_conv3x3_fwd_strip_up2(_p(x), _p(layer.wb), _p(layer.wt),
                                          _p(layer.b), _p(res), None, _p(a), n, 2 * h, 2 * w, ci,
                                          layer.cout, _s()), "sp_conv3x3_fwd_strip_up2")
     return a

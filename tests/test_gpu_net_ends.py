@@ -124,6 +124,70 @@ def test_layer_autograd(skip):
         assert rel(res.grad, rr.grad) < 4e-3
 
 
+def strided(t, how):
+    """The values of t in a tensor that is not dense (or not on 16 bytes)."""
+    if how == "permuted":
+        return t.permute(0, 3, 1, 2).contiguous().permute(0, 2, 3, 1)
+    if how == "expanded":
+        return t[:1, :1, :1].expand(t.shape)
+    buf = torch.zeros(t.numel() + 1, device="cuda", dtype=t.dtype)
+    buf[1:].copy_(t.reshape(-1))
+    return buf[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("how", ["permuted", "expanded", "off"])
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("entry", ["conv", "conv_gelu", "conv_gelu_up"])
+def test_layers_take_any_strides(entry, grad, how):
+    """Inputs and skips that are views: as the same values in dense tensors."""
+    torch.manual_seed(6)
+    n, h, w, ci, co = 2, 6, 10, 32, 64
+    up = 2 if entry == "conv_gelu_up" else 1
+    layer = S.ConvLayer(ci, co, torch.Generator().manual_seed(1))
+    x = strided(torch.randn(n, h, w, ci, device="cuda").bfloat16(), how)
+    res = strided(torch.randn(n, up * h, up * w, co, device="cuda").bfloat16(), how)
+    dy = torch.randn(n, up * h, up * w, co, device="cuda").bfloat16()
+    outs = []
+    for a, r in ((x, res), (x.clone(memory_format=torch.contiguous_format),
+                            res.clone(memory_format=torch.contiguous_format))):
+        layer.zero_grad()
+        with torch.set_grad_enabled(grad):
+            a, r = a.detach().requires_grad_(grad), r.detach().requires_grad_(grad)
+            y = getattr(S, entry)(a, layer, r)
+            if grad:
+                y.backward(dy)
+                outs.append((y.detach(), a.grad, r.grad, layer.gb.clone()))
+                wg = layer.gw.clone()
+            else:
+                outs.append((y.detach(),))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    if grad:  # (the weight gradient's sums have no fixed order)
+        first = outs[0]
+        layer.zero_grad()
+        a = x.detach().requires_grad_()
+        getattr(S, entry)(a, layer, res.detach()).backward(dy)
+        assert float((layer.gw - wg).norm() / wg.norm()) < 1e-5 and len(first) == 4
+
+
+@pytest.mark.parametrize("ch,nb", [((32, 64), 3), ((32, 64, 128), 2), ((32, 64, 128, 256), 3)])
+def test_network_down_to_one_pixel(ch, nb):
+    """A field whose deepest level is one pixel: training reads the up-sampled
+    pixel as inference does."""
+    torch.manual_seed(8)
+    net = S.JumpNet(ch, seed=2)
+    side = 2 ** (len(ch) - 1)
+    psi = torch.rand(nb, side, side, device="cuda") - 0.5
+    with torch.no_grad():
+        want = net(psi)
+    got = net(psi)
+    got.square().sum().backward()
+    # bf16 activations through two paths that round at the ends differently, and
+    # the mean of a few values taken off
+    assert torch.isfinite(got).all()
+    assert float((got.detach() - want).abs().max()) < 0.1 * float(want.abs().max()) + 1e-3
+    assert all(torch.isfinite(l.gw).all() and torch.isfinite(l.gb).all() for l in net.layers())
+
+
 @pytest.mark.parametrize("kernel", ["strip", "tc", "mma"])
 @pytest.mark.parametrize("co", [32, 128])
 def test_training_activation_is_rounded_once(kernel, co, monkeypatch):
