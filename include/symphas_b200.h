@@ -25,8 +25,9 @@
  *                (dataprocesses/datadensity.h, dataprocesses/dataenergy.h)
  *   sp_destroy   ~Model
  *
- * Threading: a handle is used by one host thread at a time; all its work runs
- * in order on one CUDA stream (its own, or the one given by sp_set_stream).
+ * Threading: a handle is used by one host thread at a time (several handles by
+ * several threads); all its work runs in order on one CUDA stream (its own, or
+ * the one given by sp_set_stream).
  * Ownership: the handle owns its device buffers; the caller owns host buffers.
  */
 #ifndef SYMPHAS_B200_H

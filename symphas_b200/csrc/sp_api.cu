@@ -885,7 +885,10 @@ int create(const sp_desc* desc, const sp_member* members, int count, sp_handle* 
   for (int i = 0; constant && i < H->batch; ++i)
     for (int f = 0; f < H->nf; ++f)
       if (int rc = refresh_halos(H, i, f)) return rc;
-  SP_CUDA(H, cudaDeviceSynchronize());
+  // the copies above ran on the default stream, the halos on the handle's own (a
+  // wait for the whole device would break a capture of another thread's handle)
+  SP_CUDA(H, cudaStreamSynchronize(nullptr));
+  SP_CUDA(H, cudaStreamSynchronize(H->stream));
   return SP_OK;
 }
 

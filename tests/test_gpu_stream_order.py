@@ -7,6 +7,8 @@ for bit, those of the same sequence run with a device synchronisation after
 every operation.
 """
 import ctypes
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -69,3 +71,40 @@ def test_foreign_kernels_between_steps_are_ordered(dim_model, dtype):
     b = _run(torch, dim_model, dtype, sync=True)
     assert np.isfinite(b).all()
     assert np.array_equal(a, b)
+
+
+def test_handles_of_several_threads():
+    """Threads that create, step (with graph captures) and destroy handles of their
+    own: a handle created while another thread captures its steps disturbs neither,
+    and the fields are those of one thread."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.set_device(0)
+
+    def field(k):
+        m = sp.model_MB_t(2, sp.SolverFT(sp.Stencil2d2h(5, 6, 13), form="fused"),
+                          sp.ProblemParameters((24 + 4 * (k % 7), 20 + k % 11)), dtype="f32")
+        m.fill_uniform(0, k, -0.3, 0.2)
+        m.step(0.01, 400)  # graph replay
+        out = m.get_field(0)
+        m.close()
+        return out
+
+    want = [field(k) for k in range(77)]
+    errors, runs, end = [], [0], time.time() + 3.0
+
+    def work(k):
+        try:
+            while time.time() < end and not errors:
+                if not np.array_equal(field(k % 77), want[k % 77]):
+                    errors.append(k)
+                k += 5
+                runs[0] += 1
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(5)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and runs[0] > 20, errors
