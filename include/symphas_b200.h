@@ -231,7 +231,11 @@ int sp_test_wait_timeout(sp_handle* h, long long cycles, int dirty_queue);
 /* Number of fused-step kernel launches issued so far by this handle. */
 long long sp_launch_count(const sp_handle* h);
 /* Device pointer of the current interior origin of a field and its
- * padded geometry (pitch and halo in elements), for zero-copy callers. */
+ * padded geometry (pitch and halo in elements), for zero-copy callers.  Who
+ * writes sites within the halo's depth of a periodic face writes their images
+ * behind the other one too: a step reads the images, or, where one launch takes
+ * several steps, the sites themselves, and the constants of the other sides from
+ * the description. */
 int sp_field_geometry(const sp_handle* h, int inst, int field, void** dev_origin,
                       long long* pitch, long long* plane, int halo[3]);
 
